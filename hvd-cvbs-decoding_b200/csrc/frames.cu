@@ -574,7 +574,7 @@ hvdg_status decode_woven_frames(hvdg_ctx* ctx, const int16_t* const* chroma,
   mark(ctx, 2);
   if (opt.do_solve) {
     const hvdg::SolverArgs sa = solver_args(ctx, S);
-    e = hvdg::launch_solver(sa, solver_grid(ctx, L.total_units, opt.ctas_per_sm), s);
+    e = launch_solve(ctx, S, sa, b.rg, false, opt.ctas_per_sm);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
     S.launches += 1;
   }

@@ -237,11 +237,11 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
   hvdg::launch_aniso(at<FieldDesc>(ctx, L.o_fields), 1, at<float2>(ctx, L.o_X0), s);
   // ---- forward, one outer per launch ----
   hvdg::SolverArgs sa = solver_args(ctx, S);
-  const int grid = solver_grid(ctx, L.total_units);
+  sa.keep_w = 1;  // each outer's weights are checkpointed
   int cg_run = 0;
   for (int o = 0; o < n_outer; ++o) {
     stage_reset(ctx, S);
-    e = hvdg::launch_solver(sa, grid, s);
+    e = launch_solve(ctx, S, sa, S.b.rg, false);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint forward solver");
     e = cudaMemcpyAsync(ck + (o + 1) * plane, at<float2>(ctx, L.o_X0), sizeof(float2) * plane,
                         cudaMemcpyDeviceToDevice, s);
@@ -317,6 +317,7 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint cotangents");
   hvdg::launch_adj_output(ag, yb, sb, cb, s);
   hvdg::SolverArgs sadj = sa;
+  sadj.keep_w = 0;
   sadj.S = zero;
   sadj.B = B;
   sadj.n_phases = fa.n_phases;
@@ -342,7 +343,7 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
     if (e == cudaSuccess) e = cudaMemsetAsync(at<float2>(ctx, L.o_X0), 0, sizeof(float2) * plane, s);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint solve setup");
     stage_reset(ctx, S);
-    e = hvdg::launch_solver(sadj, grid, s);
+    e = launch_solve(ctx, S, sadj, S.b.rg, false);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint solver");
     hvdg::AdjOuter ao;
     ao.S = at<float>(ctx, L.o_S);

@@ -44,7 +44,29 @@ struct SolverArgs {
   const float4* nbr;            // neighbour planes (S_w - S, Re dc, Im dc, conf)
   const float4* line_phasor;
   const float2* col_phasor;
+  // the resident solver (k_resident.cu)
+  const int* order;             // this launch's fields, heaviest first
+  int n_fields;
+  void* xchg;                   // kResidentXchgBytes(sm_count), zeroed before launch
+  int keep_w;                   // the last outer's weights are also left in W
 };
+
+// What the choice of solver needs to know of one field of a launch.
+struct SolveShape {
+  int h, w;
+  int n_outer, n_inner;
+};
+// Launch shape of the resident solver: `gangs` groups of `ctas` CTAs, each
+// solving one field at a time in tiles of at most `rows` rows (`nr` per warp).
+// gangs == 0: the fields do not fit on the chip (or carry the oriented prior),
+// the streaming solver takes them.
+struct ResidentPlan {
+  int gangs = 0, ctas = 0, rows = 0, nr = 0;
+};
+ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag, int sm_count);
+size_t resident_xchg_bytes(int sm_count);
+cudaError_t launch_resident(const SolverArgs& args, const ResidentPlan& plan, bool nbr,
+                            cudaStream_t st);
 
 int solver_max_blocks_per_sm(bool diag = false);
 cudaError_t launch_solver(const SolverArgs& args, int grid, cudaStream_t st);

@@ -237,6 +237,63 @@ int auto_band_rows_hw(hvdg_ctx* ctx, const std::vector<std::pair<int, int>>& hw)
   return 3;
 }
 
+// Size and solver budget of each plane (variational.cpp:224-230).
+std::vector<hvdg::SolveShape> solve_shapes(const hvdg_field_in* in, int n, const hvdg_config* cfg,
+                                           const hvdg_geometry* weave_geom) {
+  std::vector<hvdg::SolveShape> v;
+  for (int i = 0; i < (weave_geom ? n / 2 : n); ++i) {
+    const hvdg_field_in& fi = in[weave_geom ? 2 * i : i];
+    const hvdg_geometry& g = weave_geom ? *weave_geom : *fi.geometry;
+    const int outer_cfg = fi.irls_outer > 0 ? fi.irls_outer : cfg->irls_outer;
+    const int cg_cfg = fi.cg_iterations >= 0 ? fi.cg_iterations : cfg->cg_iterations;
+    hvdg::SolveShape s;
+    s.h = last_active_line(g) - g.first_active_field_line;
+    s.w = g.active_video_end - g.active_video_start;
+    s.n_outer = std::max(1, outer_cfg);
+    s.n_inner = std::max(1, (cfg->fast ? cg_cfg * 2 / 3 : cg_cfg) / s.n_outer);
+    v.push_back(s);
+  }
+  return v;
+}
+
+// The resident launches of a set of planes, one per plane size (a launch's
+// tiles all have its tallest tile's register rows, so sizes are not mixed: a
+// batch of 40 NTSC and 24 PAL fields takes 55 ms in two launches, 64 in one).
+// Empty when one of them does not fit the chip.
+std::vector<ResidentGroup> resident_groups(hvdg_ctx* ctx,
+                                           const std::vector<hvdg::SolveShape>& shapes, bool nbr,
+                                           bool diag, std::vector<int>* order) {
+  const int m = (int)shapes.size();
+  order->resize(m);
+  for (int i = 0; i < m; ++i) (*order)[i] = i;
+  auto key = [&](int i) {
+    const hvdg::SolveShape& s = shapes[i];
+    return std::make_tuple(s.h, s.w, (int64_t)s.n_outer * (s.n_inner + 3));
+  };
+  std::stable_sort(order->begin(), order->end(), [&](int i, int j) { return key(i) > key(j); });
+  std::vector<ResidentGroup> groups;
+  for (int a = 0; a < m;) {
+    int b = a;
+    std::vector<hvdg::SolveShape> part;
+    while (b < m && shapes[(*order)[b]].h == shapes[(*order)[a]].h &&
+           shapes[(*order)[b]].w == shapes[(*order)[a]].w)
+      part.push_back(shapes[(*order)[b++]]);
+    ResidentGroup g;
+    g.plan = hvdg::plan_resident(part.data(), b - a, nbr, diag, ctx->sm_count);
+    g.off = a;
+    g.n = b - a;
+    if (!g.plan.gangs) return {};
+    groups.push_back(g);
+    a = b;
+  }
+  return groups;
+}
+
+// A tiling set on the context or for the call is the streaming solver's.
+bool resident_allowed(const hvdg_ctx* ctx, int band_rows, int ctas) {
+  return band_rows <= 0 && ctas <= 0 && ctx->band_rows <= 0 && ctx->ctas_per_sm <= 0;
+}
+
 int auto_band_rows(hvdg_ctx* ctx, const std::vector<FieldPlan>& fp) {
   std::vector<std::pair<int, int>> hw;
   for (const FieldPlan& p : fp) hw.emplace_back(p.h, p.w);
@@ -334,12 +391,17 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
     b.gcol_off.push_back(ncol);
     ncol += t.w;
   }
+  // the resident solver wherever the planes fit (a tiling set by the caller
+  // or the tuner belongs to the streaming one); it takes no units
+  const std::vector<hvdg::SolveShape> shapes = solve_shapes(in, n, cfg, weave_geom);
+  b.order.assign(m, 0);
+  if (resident_allowed(ctx, band_rows))
+    b.rg = resident_groups(ctx, shapes, false, cfg->diag_prior > 0.0f, &b.order);
   // per-field descriptors, units
-  const int band = band_rows > 0 ? band_rows : auto_band_rows(ctx, b.fp);
+  const int band = band_rows > 0 ? band_rows : !b.rg.empty() ? 32 : auto_band_rows(ctx, b.fp);
   for (int i = 0; i < m; ++i) {
     const FieldPlan& p = b.fp[i];
     const hvdg_geometry& g = *p.g;
-    const hvdg_field_in& fi = in[weave_geom ? 2 * i : i];
     FieldDesc f;
     std::memset(&f, 0, sizeof(f));
     f.h = p.h;
@@ -352,12 +414,8 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
     f.col_off = b.gcol_off[p.geom_slot];
     f.geom = p.geom_slot;
     f.is_pal = uses_vswitch(g) ? 1 : 0;
-    // solver budget (variational.cpp:224-230)
-    const int outer_cfg = fi.irls_outer > 0 ? fi.irls_outer : cfg->irls_outer;
-    const int cg_cfg = fi.cg_iterations >= 0 ? fi.cg_iterations : cfg->cg_iterations;
-    f.n_outer = std::max(1, outer_cfg);
-    const int cg_total = cfg->fast ? cg_cfg * 2 / 3 : cg_cfg;
-    f.n_inner = std::max(1, cg_total / f.n_outer);
+    f.n_outer = shapes[i].n_outer;
+    f.n_inner = shapes[i].n_inner;
     f.cg_tol = cfg->cg_tol > 0.0f ? cfg->cg_tol : (cfg->fast ? 0.10f : 0.02f);
     f.eps = cfg->charbonnier_eps;
     f.eps_c = cfg->chroma_eps;
@@ -473,6 +531,7 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
   L.o_arrive = take(sizeof(int) * m);
   L.o_flags = take(sizeof(int) * 4);
   L.o_queue = take(sizeof(unsigned long long));
+  L.o_order = take(sizeof(int) * m);
   L.o_lineph = take(sizeof(float4) * lines);
   L.o_theta = take(sizeof(float) * theta);
   L.o_theta64 = take(sizeof(double) * theta);
@@ -501,6 +560,7 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
   for (const FieldDesc& f : b.fields) L.has_diag |= f.diag_prior > 0.0f;
   L.o_W2 = L.has_diag ? take(sizeof(float2) * px) : 0;
   L.o_rowbuf = take(sizeof(float2) * rowb);
+  L.o_xchg = take(hvdg::resident_xchg_bytes(ctx->sm_count));
   L.total = o;
   return HVDG_OK;
 }
@@ -598,6 +658,7 @@ hvdg_status stage_upload(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hv
   put(L.o_fields, b.fields.data(), sizeof(FieldDesc) * m);
   put(L.o_geoms, b.geoms.data(), sizeof(GeomDesc) * b.geoms.size());
   put(L.o_units, b.units.data(), sizeof(Unit) * b.units.size());
+  put(L.o_order, b.order.data(), sizeof(int) * m);
   {
     std::vector<int> done(m, -1);
     put(L.o_done, done.data(), sizeof(int) * m);
@@ -799,6 +860,28 @@ int solver_grid(hvdg_ctx* ctx, int n_units, int ctas_override) {
                                         (hvdg::kSolverThreads / 32)));
 }
 
+// The solve of a batch: the resident launches of `groups`, or, when there are
+// none, streaming over sa's units (the caller has reset its control state).
+cudaError_t launch_solve(hvdg_ctx* ctx, const Staged& S, const hvdg::SolverArgs& sa,
+                         const std::vector<ResidentGroup>& groups, bool nbr, int ctas_override) {
+  if (groups.empty())
+    return hvdg::launch_solver(sa, solver_grid(ctx, sa.n_units, ctas_override), ctx->stream);
+  for (const ResidentGroup& g : groups) {
+    hvdg::SolverArgs a = sa;
+    a.order = at<int>(ctx, S.b.L.o_order) + g.off;
+    a.n_fields = g.n;
+    a.xchg = at<char>(ctx, S.b.L.o_xchg);
+    cudaError_t e = cudaMemsetAsync(a.xchg, 0,
+                                    hvdg::resident_xchg_bytes(g.plan.gangs * g.plan.ctas),
+                                    ctx->stream);
+    if (e == cudaSuccess && g.n > g.plan.gangs)
+      e = cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), ctx->stream);
+    if (e == cudaSuccess) e = hvdg::launch_resident(a, g.plan, nbr, ctx->stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 // Copy the outputs, read the flags, synchronise, fill the diagnostics.
 hvdg_status stage_finish(hvdg_ctx* ctx, Staged& S, hvdg_field_out* out, const RunOpts& opt,
                          hvdg_diag* diag) {
@@ -885,7 +968,7 @@ hvdg_status run_batch_once(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const 
   if (opt.do_solve) {
     const hvdg::SolverArgs sa = solver_args(ctx, S);
     const cudaError_t e =
-        hvdg::launch_solver(sa, solver_grid(ctx, L.total_units, opt.ctas_per_sm), s);
+        launch_solve(ctx, S, sa, S.b.rg, false, opt.ctas_per_sm);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
     S.launches += 1;
   }
@@ -959,7 +1042,7 @@ hvdg_status run_batch_graph(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const
       hvdg::launch_aniso(at<FieldDesc>(ctx, L.o_fields), n, at<float2>(ctx, L.o_X0), s);
       mark(ctx, 2);
       const hvdg::SolverArgs sa = solver_args(ctx, S);
-      e = hvdg::launch_solver(sa, solver_grid(ctx, L.total_units, opt.ctas_per_sm), s);
+      e = launch_solve(ctx, S, sa, S.b.rg, false, opt.ctas_per_sm);
       if (e != cudaSuccess) st = hvdg::cuda_fail(ctx, e, "solver launch");
       mark(ctx, 3);
     }
@@ -1045,14 +1128,21 @@ hvdg_status graph_result(hvdg_ctx* ctx, hvdg_diag* diag) {
   return HVDG_OK;
 }
 
-// Batched decode: autotune the solver tiling once per batch signature (band
+static bool resident_fits(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg_config* cfg) {
+  std::vector<int> order;
+  return resident_allowed(ctx) &&
+         !resident_groups(ctx, solve_shapes(in, n, cfg), false, cfg->diag_prior > 0.0f, &order)
+              .empty();
+}
+
+// Batched decode: autotune the streaming solver's tiling once per batch signature (band
 // height x CTAs per SM, timed on the solver's own events), then run -- as a
 // replayed CUDA graph when the buffers are device-resident.
 hvdg_status run_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg_config* cfg,
                       hvdg_field_out* out, hvdg_diag* diag, const RunOpts& opt_in) {
   RunOpts opt = opt_in;
   if (opt.do_solve && opt.do_init && opt.do_lockin && !opt.amp_out && ctx->autotune &&
-      ctx->band_rows == 0 && ctx->ctas_per_sm == 0 && n >= 8) {
+      ctx->band_rows == 0 && ctx->ctas_per_sm == 0 && n >= 8 && !resident_fits(ctx, in, n, cfg)) {
     const std::string sig = batch_signature(in, n, cfg);
     auto it = ctx->tune.find(sig);
     if (it == ctx->tune.end()) {

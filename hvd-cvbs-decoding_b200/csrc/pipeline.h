@@ -187,6 +187,7 @@ struct Layout {
       o_amp;
   size_t o_W2 = 0;   // (wd1, wd2) plane, only when a field has the oriented prior
   size_t o_gpart = 0, o_garrive = 0;  // solver unit-group partials and arrival counters
+  size_t o_order = 0, o_xchg = 0;     // resident solver: field order, exchange slots
   bool has_diag = false;
   size_t total;
   int64_t total_px, total_rowbuf;
@@ -195,6 +196,13 @@ struct Layout {
 };
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// Planes of one size, solved by one resident launch: `n` entries of the order
+// table from `off` on.
+struct ResidentGroup {
+  hvdg::ResidentPlan plan;
+  int off, n;
+};
 
 struct Batch {
   std::vector<FieldPlan> fp;
@@ -214,6 +222,8 @@ struct Batch {
   // per field: the solver writes luma / chroma straight to the caller's
   // buffers (FieldDesc out_y / out_c), so no copy follows
   std::vector<char> direct_y, direct_c;
+  std::vector<int> order;    // planes by size, then by solver work, heaviest first
+  std::vector<ResidentGroup> rg;  // empty: the streaming solver takes the batch
   Layout L;
   int max_phases = 0;
 };
@@ -293,6 +303,15 @@ hvdg::InitArgs init_args(hvdg_ctx* ctx, const Staged& S);
 hvdg_status stage_prepare(hvdg_ctx* ctx, Staged& S, const RunOpts& opt);
 hvdg::SolverArgs solver_args(hvdg_ctx* ctx, const Staged& S);
 int solver_grid(hvdg_ctx* ctx, int n_units, int ctas_override = -1);
+std::vector<hvdg::SolveShape> solve_shapes(const hvdg_field_in* in, int n, const hvdg_config* cfg,
+                                           const hvdg_geometry* weave_geom = nullptr);
+bool resident_allowed(const hvdg_ctx* ctx, int band_rows = -1, int ctas = -1);
+cudaError_t launch_solve(hvdg_ctx* ctx, const Staged& S, const hvdg::SolverArgs& sa,
+                         const std::vector<ResidentGroup>& groups, bool nbr,
+                         int ctas_override = -1);
+std::vector<ResidentGroup> resident_groups(hvdg_ctx* ctx,
+                                           const std::vector<hvdg::SolveShape>& shapes, bool nbr,
+                                           bool diag, std::vector<int>* order);
 hvdg_status stage_finish(hvdg_ctx* ctx, Staged& S, hvdg_field_out* out, const RunOpts& opt,
                          hvdg_diag* diag);
 hvdg_status run_batch_once(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg_config* cfg,

@@ -308,8 +308,19 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
   }
   // units regrouped by colour (each field's units stay contiguous)
   std::vector<Unit> cunits;
-  std::vector<int> cbegin, ccount, cphases;
+  std::vector<int> cbegin, ccount, cphases, corder;
+  std::vector<std::vector<ResidentGroup>> crg;
+  const std::vector<hvdg::SolveShape> shapes = solve_shapes(in, nf, &cfg);
   for (const auto& col : colors) {
+    // all fields of a window share their geometry and budget
+    ResidentGroup rg;
+    rg.off = (int)corder.size();
+    rg.n = (int)col.size();
+    corder.insert(corder.end(), col.begin(), col.end());
+    if (resident_allowed(ctx))
+      rg.plan = hvdg::plan_resident(shapes.data(), rg.n, has_temporal, cfg.diag_prior > 0.0f,
+                                    ctx->sm_count);
+    crg.push_back(rg.plan.gangs ? std::vector<ResidentGroup>{rg} : std::vector<ResidentGroup>());
     cbegin.push_back((int)cunits.size());
     int ph = 0;
     for (int j : col) {
@@ -334,6 +345,9 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
   }
   e = cudaMemcpyAsync(at<Unit>(ctx, L.o_units), cunits.data(), sizeof(Unit) * cunits.size(),
                       cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(at<int>(ctx, L.o_order), corder.data(), sizeof(int) * corder.size(),
+                        cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "H2D units");
   hvdg::SolverArgs sa = solver_args(ctx, S);
   sa.M = at<float4>(ctx, X(x_M));
@@ -710,7 +724,7 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
         sa.unit_base = cbegin[ci];
         sa.n_units = ccount[ci];
         sa.n_phases = cphases[ci];
-        e = hvdg::launch_solver(sa, solver_grid(ctx, ccount[ci]), s);
+        e = launch_solve(ctx, S, sa, crg[ci], has_temporal);
         if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
         S.launches += 2;
       }
