@@ -17,6 +17,7 @@
 
 #include "hvdg_common.cuh"
 #include "k_temporal.h"
+#include "per_device.h"
 
 namespace hvdg {
 
@@ -79,82 +80,70 @@ __global__ void k_env_maps(const FieldDesc* __restrict__ fields, const int* __re
 }
 
 // (2) smooth_rows (sequence.cpp:860-889): sliding sum over [x-2, x+2] clipped
-// to the row, sqrt(mean), both maps. The running sums: one warp per (field,
-// 32-row band, map): lane l runs row l's in-order float running sum (the
-// same additions and subtractions in column order); the band's samples
-// arrive 32 columns (plus the window's 3 / 2 columns either side) at a time
-// through shared memory, one coalesced row segment per load instruction, and
-// the sums leave the same way. The tile's rows are 41 floats apart, so a
-// lane's reads along its row hit a different bank from every other lane's.
-// The means and square roots, off the chain, follow in k_env_sqrt.
-__global__ void k_env_smooth(const FieldDesc* __restrict__ fields, const int* __restrict__ list,
-                             const float* __restrict__ gmag, const float* __restrict__ lapmag,
-                             float* __restrict__ vraw, float* __restrict__ traw) {
-  __shared__ float tile[32][41];
+// to the row, sqrt(mean), both maps. The running sum is a float chain in
+// column order (one addition and one subtraction per column); a block takes an
+// 8-row band of one map into shared memory (all its warps, coalesced), one lane
+// per row runs the chain, and all warps write the roots of the means. Slot x
+// of a row holds sample x - 3 (zeros outside the row, which leave the sum as it
+// is) and then column x's sum: no later column reads it. Two kernels (a warp
+// per 32 rows staging and summing in turn, then the roots) took 94 us for two
+// NTSC fields, this 9.
+constexpr int kSmoothRows = 8;
+__host__ __device__ constexpr int smooth_stride(int w) { return (w + 5) | 1; }
+__global__ void __launch_bounds__(256) k_env_smooth(const FieldDesc* __restrict__ fields,
+                                                    const int* __restrict__ list,
+                                                    const float* __restrict__ gmag,
+                                                    const float* __restrict__ lapmag,
+                                                    float* __restrict__ vraw,
+                                                    float* __restrict__ traw) {
+  extern __shared__ float smooth_smem[];
   const FieldDesc f = fields[list[blockIdx.y]];
-  const int y0 = blockIdx.x * 32;
+  const int y0 = blockIdx.x * kSmoothRows;
   if (y0 >= f.h) return;
-  const int lane = threadIdx.x & 31;
-  const int rows = min(32, f.h - y0);
-  const bool live = lane < rows;
-  const int ww = f.w;
-  const int m = blockIdx.z;
-  const float* src = (m == 0 ? gmag : lapmag) + f.px_off + (int64_t)y0 * f.pitch;
-  float* out = (m == 0 ? vraw : traw) + f.px_off + (int64_t)y0 * f.pitch;
-  float acc = 0.0f;
-  if (live)
-    for (int x = 0; x < (ww < 3 ? ww : 3); ++x) acc += src[(int64_t)lane * f.pitch + x];
-  for (int c0 = 0; c0 < ww; c0 += 32) {
-    // columns c0 - 3 .. c0 + 34 of every row of the band
-    {
-      // all loads issued before the first store
-      float v[32], e[32];
-      const int col = c0 - 3 + lane, col2 = c0 + 29 + lane;  // second pass: lanes 0-5
-      const bool in1 = col >= 0 && col < ww, in2 = lane < 6 && col2 < ww;
-#pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        v[q] = in1 && q < rows ? src[(int64_t)q * f.pitch + col] : 0.0f;
-        e[q] = in2 && q < rows ? src[(int64_t)q * f.pitch + col2] : 0.0f;
-      }
-#pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        tile[q][lane] = v[q];
-        if (lane < 6) tile[q][32 + lane] = e[q];
-      }
-    }
-    __syncwarp();
-    const int mm = min(32, ww - c0);  // columns of this chunk
-    // column j reads tile columns j and j + 5 and then holds its running
-    // sum in column j (no later column reads it)
-    for (int j = 0; j < mm; ++j) {
-      const int x = c0 + j;
-      if (x > 0) {
-        if (x + 2 < ww) acc += tile[lane][j + 5];
-        if (x - 3 >= 0) acc -= tile[lane][j];
-      }
-      tile[lane][j] = acc;
-    }
-    __syncwarp();
-#pragma unroll 4
-    for (int q = 0; q < rows; ++q)
-      if (lane < mm) out[(int64_t)q * f.pitch + c0 + lane] = tile[q][lane];
-    __syncwarp();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rows = min(kSmoothRows, f.h - y0), w = f.w, stride = smooth_stride(w);
+  const int64_t o = f.px_off + (int64_t)(y0 + warp) * f.pitch;
+  float* b = smooth_smem + warp * stride;
+  if (warp < rows) {
+    const float* src = (blockIdx.z == 0 ? gmag : lapmag) + o;
+#pragma unroll 8
+    for (int x = lane; x < w + 5; x += 32) b[x] = x >= 3 && x < w + 3 ? src[x - 3] : 0.0f;
   }
-}
-
-// (2b) the running sums to sqrt(sum / taps), taps = |[x-2, x+2] clipped to
-// the row|, both maps, one thread per pixel
-__global__ void k_env_sqrt(const FieldDesc* __restrict__ fields, const int* __restrict__ list,
-                           float* __restrict__ vraw, float* __restrict__ traw) {
-  const FieldDesc f = fields[list[blockIdx.z]];
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y;
-  if (x >= f.w || y >= f.h) return;
-  const int lo = x - 2, hi = x + 2;
-  const int n_taps = (hi < f.w - 1 ? hi : f.w - 1) - (lo > 0 ? lo : 0) + 1;
-  const int64_t o = f.px_off + (int64_t)y * f.pitch + x;
-  vraw[o] = sqrtf(vraw[o] / (float)n_taps);
-  traw[o] = sqrtf(traw[o] / (float)n_taps);
+  __syncthreads();
+  if (threadIdx.x < rows) {
+    float* c = smooth_smem + threadIdx.x * stride;
+    float acc = 0.0f;
+    for (int x = 0; x < (w < 3 ? w : 3); ++x) acc += c[x + 3];
+    c[0] = acc;
+    int x = 1;
+    for (; x + 16 <= w; x += 16) {
+      float in[16], out[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        in[k] = c[x + k + 5];
+        out[k] = c[x + k];
+      }
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        acc += in[k];
+        acc -= out[k];
+        c[x + k] = acc;
+      }
+    }
+    for (; x < w; ++x) {
+      acc += c[x + 5];
+      acc -= c[x];
+      c[x] = acc;
+    }
+  }
+  __syncthreads();
+  if (warp < rows) {
+    float* dst = (blockIdx.z == 0 ? vraw : traw) + o;
+    for (int x = lane; x < w; x += 32) {
+      const int n_taps = min(x + 2, w - 1) - max(x - 2, 0) + 1;
+      dst[x] = sqrtf(b[x] / (float)n_taps);
+    }
+  }
 }
 
 // (3) median of every 7th envelope value (flat row-major index), per field
@@ -182,7 +171,28 @@ __global__ void __launch_bounds__(1024) k_env_floor(const FieldDesc* __restrict_
   if (n > 0) {
     med = block_select_kth(smp, n, n / 2, hist, bc);
     if (n % 2 == 0) {
-      const float lo = block_select_kth(smp, n, n / 2 - 1, hist, bc);
+      // the value of rank n/2 - 1: the largest one below med when exactly n/2 lie
+      // below it, else med itself (one pass instead of a second selection)
+      __shared__ unsigned below, top;
+      if (threadIdx.x == 0) below = top = 0;
+      __syncthreads();
+      const unsigned key = float_key(med);
+      unsigned cnt = 0, mx = 0;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const unsigned k = float_key(smp[i]);
+        if (k < key) {
+          ++cnt;
+          mx = max(mx, k);
+        }
+      }
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if ((threadIdx.x & 31) == 0 && cnt) {
+        atomicAdd(&below, cnt);
+        atomicMax(&top, mx);
+      }
+      __syncthreads();
+      const float lo = below == (unsigned)(n / 2) ? key_float(top) : med;
       med = 0.5f * (med + lo);
     }
   }
@@ -375,10 +385,14 @@ void launch_envelope(const FieldDesc* d_fields, const int* d_list, int n, int ma
   if (n <= 0) return;
   k_env_maps<<<dim3((max_w + 127) / 128, max_h, n), 128, 0, st>>>(d_fields, d_list, Y, X, e.gmag,
                                                                    e.lapmag);
-  k_env_smooth<<<dim3((max_h + 31) / 32, n, 2), 32, 0, st>>>(d_fields, d_list, e.gmag, e.lapmag,
-                                                             e.vraw, e.traw);
-  k_env_sqrt<<<dim3((max_w + 127) / 128, max_h, n), 128, 0, st>>>(d_fields, d_list, e.vraw,
-                                                                   e.traw);
+  static PerDeviceOnce once;
+  once([] {
+    // rows of up to 2048 samples
+    cudaFuncSetAttribute(k_env_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 << 10);
+  });
+  k_env_smooth<<<dim3((max_h + kSmoothRows - 1) / kSmoothRows, n, 2), 256,
+                 sizeof(float) * kSmoothRows * smooth_stride(max_w), st>>>(
+      d_fields, d_list, e.gmag, e.lapmag, e.vraw, e.traw);
   k_env_floor<<<n, 1024, 0, st>>>(d_fields, d_list, e.vraw, e.scratch, e.scratch_off, e.floor2);
   k_env_gate<<<dim3((max_w + 127) / 128, max_h, n), 128, 0, st>>>(
       d_fields, d_list, e.vraw, e.traw, e.floor2, e2, floor_max, e.gate);
