@@ -92,7 +92,6 @@ hvdg_status estimate_motion_sad(hvdg_ctx* ctx, const float* y_ref, const float* 
   const size_t o_f = take(sizeof(hvdg::MeField) * 2);
   const size_t o_p = take(sizeof(hvdg::MePair));
   const size_t o_l = take(sizeof(float) * 2 * plane);
-  const size_t o_v = take(sizeof(int) * 2 * plane);
   const size_t o_q = take(sizeof(int) * 2 * plane);
   size_t of[7], od[4];
   for (int i = 0; i < 7; ++i) of[i] = take(sizeof(float) * nt);
@@ -127,7 +126,6 @@ hvdg_status estimate_motion_sad(hvdg_ctx* ctx, const float* y_ref, const float* 
   a.tiles_off = nt;
   hvdg::SadBuffers b;
   b.luma = reinterpret_cast<const float*>(base + o_l);
-  b.vsum = reinterpret_cast<int*>(base + o_v);
   b.qblur = reinterpret_cast<int*>(base + o_q);
   b.mdy = reinterpret_cast<float*>(base + of[0]);
   b.mdx = reinterpret_cast<float*>(base + of[1]);

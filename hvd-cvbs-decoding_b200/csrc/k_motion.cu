@@ -26,233 +26,158 @@ namespace hvdg {
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// One line of BoxBlur (motion.cpp:21-55): prefix sums c_k = c_(k-1) +
-// s_(k-1) in double, in order, and out_i = (c_min(i+r+1, n) - c_max(i-r, 0))
-// * norm; samples `ss` apart in the source, outputs `ds` apart. Output i is
-// written as soon as the prefix its window ends at exists (the ones cut by
-// the line's end last). The last 32 prefix sums of each thread live in a
-// shared-memory history (slot k & 31, one column per thread of a block of
-// at most kBoxThreads), so no step divides or touches local memory; the
-// samples are fetched kBoxChunk at a time ahead of their additions. The
-// values are those of the sample-by-sample loop. Needs 2 r + 1 <= 31.
-constexpr int kBoxChunk = 16;
-constexpr int kBoxThreads = 128;
+// BoxBlur (motion.cpp:21-55): prefix sums c_k = c_(k-1) + s_(k-1) of a line in
+// double, in order, and out_i = (c_min(i+r+1, n) - c_max(i-r, 0)) * norm. The
+// order of the additions is the reference's, so a line is one serial chain of
+// double additions (~10 cycles each, 4 us for a 760-sample row) and nothing
+// else should be serial: a block takes a band of whole lines into shared
+// memory as doubles (all its warps, coalesced), one lane per line runs the
+// chain in place, kChain values ahead of their additions, and all warps form
+// the window sums from the prefixes. Bands of 8 rows or 16 columns keep many
+// blocks in flight. A band is read whole before it is written, so source and
+// destination may be the same plane. Against a warp that staged, chained and
+// windowed 32 rows in turn (and a thread per column), 760 x 242, two planes:
+// rows 72 -> 11 us, columns 46 -> 7 us.
+constexpr int kBoxThreads = 256;
+constexpr int kRowBand = 8;
+constexpr int kColBand = 16;
+constexpr int kChain = 16;
 
-__device__ __forceinline__ void box_line(const float* __restrict__ s, int64_t ss,
-                                         float* __restrict__ d, int64_t ds, int n, int r,
-                                         double norm) {
-  __shared__ double hist[32 * kBoxThreads];
-  double* h = hist + threadIdx.x;
-  double c = 0.0;
-  for (int k0 = 1; k0 <= n; k0 += kBoxChunk) {
-    float v[kBoxChunk];
+__host__ __device__ constexpr int row_stride(int n) { return (n + 1) | 1; }
+constexpr size_t kBoxSmem = 200 << 10;
+
+// c[ss], c[2 ss], ... c[n ss] <- their prefix sums; c[0] <- 0.
+__device__ __forceinline__ void chain_line(double* c, int ss, int n) {
+  double acc = 0.0;
+  c[0] = 0.0;
+  int k = 1;
+  for (; k + kChain <= n + 1; k += kChain) {
+    double v[kChain];
 #pragma unroll
-    for (int j = 0; j < kBoxChunk; ++j) v[j] = k0 + j <= n ? s[(int64_t)(k0 - 1 + j) * ss] : 0.0f;
+    for (int j = 0; j < kChain; ++j) v[j] = c[(k + j) * ss];
 #pragma unroll
-    for (int j = 0; j < kBoxChunk; ++j) {
-      const int k = k0 + j;
-      if (k <= n) {
-        c = c + (double)v[j];
-        h[(k & 31) * kBoxThreads] = c;
-        const int i = k - r - 1;
-        if (i >= 0) {
-          const int i0 = i - r;
-          const double c0v = i0 > 0 ? h[(i0 & 31) * kBoxThreads] : 0.0;
-          d[(int64_t)i * ds] = (float)((c - c0v) * norm);
-        }
-      }
+    for (int j = 0; j < kChain; ++j) {
+      acc = acc + v[j];
+      c[(k + j) * ss] = acc;
     }
   }
-  for (int i = n - r > 0 ? n - r : 0; i < n; ++i) {
-    const int i0 = i - r;
-    d[(int64_t)i * ds] = (float)((c - (i0 > 0 ? h[(i0 & 31) * kBoxThreads] : 0.0)) * norm);
+  for (; k <= n; ++k) {
+    acc = acc + c[k * ss];
+    c[k * ss] = acc;
   }
 }
 
-// Shared memory of the row blur (declared once per kernel): the band's
-// 32 x 32 sample / output tile and each lane's 64-slot prefix history.
-struct RowBlurSmem {
-  float tile[32][33];
-  double hist[32][65];
-};
-
-// box_line along rows for one warp: lane l runs row l of a 32-row band
-// (`rows` of them exist). The band's samples arrive 32 columns at a time
-// through shared memory, each load instruction reading one row's 32
-// consecutive columns. Per chunk, each lane first runs its row's prefix sums
-// (the only serial chain: one double add per column, in column order, the
-// loads and conversions ahead of it) into a 64-slot shared-memory history,
-// then forms the chunk's window sums from that history with no chain at all
-// (prefix k minus prefix k - 2 r - 1, the same doubles as a running ring),
-// and the outputs leave through a shared tile as coalesced row segments.
-// Needs 2 r + 1 <= 32.
-__device__ __forceinline__ void box_rows_warp_any(RowBlurSmem& sm, const float* __restrict__ s,
-                                                  float* __restrict__ d, int64_t pitch, int rows,
-                                                  int n, int r, double norm) {
-  float (&tile)[32][33] = sm.tile;
-  double (&pre)[32][65] = sm.hist;  // prefix k of lane l at pre[l][k & 63]
-  const int lane = threadIdx.x & 31;
-  double* hist = pre[lane];
-  double c = 0.0;
-  hist[0] = 0.0;
-  for (int c0 = 0; c0 < n; c0 += 32) {
-    {
-      // all 32 loads issued before the first store
-      float v[32];
-      const bool col = c0 + lane < n;
-#pragma unroll
-      for (int q = 0; q < 32; ++q) v[q] = col && q < rows ? s[(int64_t)q * pitch + c0 + lane] : 0.0f;
-#pragma unroll
-      for (int q = 0; q < 32; ++q) tile[q][lane] = v[q];
-    }
-    __syncwarp();
-    const int m = min(32, n - c0);  // columns of this chunk
-    {
-      double v[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (double)tile[lane][j];
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < m) {
-          c = c + v[j];
-          hist[(c0 + j + 1) & 63] = c;
-        }
-    }
-    __syncwarp();
-    // window sums ending at prefix k = c0 + j + 1: output column i = k - r - 1
-    // (window [max(i - r, 0), i + r]), staged in the tile at column j
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int k = c0 + j + 1, i = k - r - 1;
-      float o = 0.0f;
-      if (j < m && i >= 0) {
-        const double c0v = i - r > 0 ? hist[(i - r) & 63] : 0.0;
-        o = (float)((hist[k & 63] - c0v) * norm);
-      }
-      tile[lane][j] = o;
-    }
-    __syncwarp();
-    // row q's outputs of this chunk: columns c0 - r .. c0 + m - 1 - r
+// `rows` (<= kRowBand) rows of n samples.
+__device__ __forceinline__ void box_rows(const float* s, float* d, int64_t pitch, int rows,
+                                         int n, int r, double norm) {
+  extern __shared__ double box_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int stride = row_stride(n);
+  double* pre = box_smem + warp * stride;
+  if (warp < rows) {
+    const float* row = s + (int64_t)warp * pitch;
+#pragma unroll 8
+    for (int x = lane; x < n; x += 32) pre[x + 1] = (double)row[x];
+  }
+  __syncthreads();
+  if (threadIdx.x < rows) chain_line(box_smem + threadIdx.x * stride, 1, n);
+  __syncthreads();
+  if (warp < rows) {
+    float* row = d + (int64_t)warp * pitch;
 #pragma unroll 4
-    for (int q = 0; q < rows; ++q) {
-      const int i = c0 - r + lane;
-      if (lane < m && i >= 0) d[(int64_t)q * pitch + i] = tile[q][lane];
+    for (int i = lane; i < n; i += 32) {
+      const double hi = pre[i + r + 1 < n ? i + r + 1 : n], lo = pre[i - r > 0 ? i - r : 0];
+      row[i] = (float)((hi - lo) * norm);
     }
-    __syncwarp();
-  }
-  if (lane >= rows) return;
-  // outputs whose window is cut by the end: prefix n is c
-  float* drow = d + (int64_t)lane * pitch;
-  for (int i = n - r > 0 ? n - r : 0; i < n; ++i) {
-    const int i0 = i - r > 0 ? i - r : 0;
-    drow[i] = (float)((c - (i0 > 0 ? hist[i0 & 63] : 0.0)) * norm);
   }
 }
 
-// The same blur for a radius known at compile time (the window's 2, 6 and
-// 8): a chunk's prefix sums and the previous chunk's stay in registers (every
-// index is a constant), so a column costs its one chained addition, a copy
-// of the sum into a shared history (read only by the windows cut by the
-// row's end) and its window sum.
-template <int R>
-__device__ __forceinline__ void box_rows_warp_r(RowBlurSmem& sm, const float* __restrict__ s,
-                                                float* __restrict__ d, int64_t pitch, int rows,
-                                                int n, double norm) {
-  constexpr int kW = 2 * R + 1;  // window: prefix k minus prefix k - kW
-  static_assert(kW <= 32, "window within two chunks");
-  float (&tile)[32][33] = sm.tile;
-  double (&hist)[32][65] = sm.hist;
-  const int lane = threadIdx.x & 31;
-  double* hrow = hist[lane];  // prefix k at slot k & 63, for the cut windows
-  double c = 0.0, prev[32], cur[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j) prev[j] = 0.0;
-  for (int c0 = 0; c0 < n; c0 += 32) {
-    {
-      float v[32];
-      const bool col = c0 + lane < n;
-#pragma unroll
-      for (int q = 0; q < 32; ++q) v[q] = col && q < rows ? s[(int64_t)q * pitch + c0 + lane] : 0.0f;
-#pragma unroll
-      for (int q = 0; q < 32; ++q) tile[q][lane] = v[q];
-    }
-    __syncwarp();
-    const int m = min(32, n - c0);
-    // the chain: cur[j] = prefix c0 + j + 1, in column order
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float x = tile[lane][j];
-      if (j < m) {
-        c = c + (double)x;
-        hrow[(c0 + j + 1) & 63] = c;
-      }
-      cur[j] = c;
-    }
-    __syncwarp();
-    // window sums ending at prefix k = c0 + j + 1 (output column k - R - 1),
-    // starting at prefix k - kW (0 below 1)
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int k = c0 + j + 1, i = k - R - 1;
-      const double c0v = k - kW > 0 ? (j - kW >= 0 ? cur[j - kW] : prev[j - kW + 32]) : 0.0;
-      tile[lane][j] = (j < m && i >= 0) ? (float)((cur[j] - c0v) * norm) : 0.0f;
-    }
-    __syncwarp();
+// `cols` (<= kColBand) columns of n samples.
+__device__ __forceinline__ void box_cols(const float* s, float* d, int64_t pitch, int band,
+                                         int cols, int n, int r, double norm) {
+  extern __shared__ double box_smem[];
+  const int x = threadIdx.x % band, y0 = threadIdx.x / band, step = kBoxThreads / band;
+  if (x < cols) {
+#pragma unroll 8
+    for (int y = y0; y < n; y += step)
+      box_smem[(y + 1) * band + x] = (double)s[(int64_t)y * pitch + x];
+  }
+  __syncthreads();
+  if (threadIdx.x < cols) chain_line(box_smem + threadIdx.x, band, n);
+  __syncthreads();
+  if (x < cols) {
 #pragma unroll 4
-    for (int q = 0; q < rows; ++q) {
-      const int i = c0 - R + lane;
-      if (lane < m && i >= 0) d[(int64_t)q * pitch + i] = tile[q][lane];
+    for (int y = y0; y < n; y += step) {
+      const double hi = box_smem[(y + r + 1 < n ? y + r + 1 : n) * band + x];
+      const double lo = box_smem[(y - r > 0 ? y - r : 0) * band + x];
+      d[(int64_t)y * pitch + x] = (float)((hi - lo) * norm);
     }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 32; ++j) prev[j] = cur[j];
-  }
-  if (lane >= rows) return;
-  // the windows cut by the row's end start within the last 2 R prefixes
-  float* drow = d + (int64_t)lane * pitch;
-  for (int i = n - R > 0 ? n - R : 0; i < n; ++i) {
-    const int i0 = i - R;
-    drow[i] = (float)((c - (i0 > 0 ? hrow[i0 & 63] : 0.0)) * norm);
   }
 }
 
-__device__ __forceinline__ void box_rows_warp(const float* __restrict__ s, float* __restrict__ d,
-                                              int64_t pitch, int rows, int n, int r,
-                                              double norm) {
-  __shared__ RowBlurSmem sm;
-  if (r == 2) return box_rows_warp_r<2>(sm, s, d, pitch, rows, n, norm);
-  if (r == 6) return box_rows_warp_r<6>(sm, s, d, pitch, rows, n, norm);
-  if (r == 8) return box_rows_warp_r<8>(sm, s, d, pitch, rows, n, norm);
-  box_rows_warp_any(sm, s, d, pitch, rows, n, r, norm);
+// A line too long for shared memory (more than ~25,000 samples): one thread,
+// the last 32 prefixes in a ring (2 r + 1 <= 31). Not in place.
+__device__ void box_line_long(const float* s, float* d, int64_t ss, int n, int r, double norm) {
+  double ring[32], c = 0.0;
+  ring[0] = 0.0;
+  for (int k = 1; k <= n + r; ++k) {
+    if (k <= n) {
+      c = c + (double)s[(int64_t)(k - 1) * ss];
+      ring[k & 31] = c;
+    }
+    const int i = k - r - 1;
+    if (i >= 0) d[(int64_t)i * ss] = (float)((c - (i - r > 0 ? ring[(i - r) & 31] : 0.0)) * norm);
+  }
 }
 
-// ---- BoxBlur (motion.cpp:21-55): double prefix sums, constant 1/(2r+1) ----
-// Vertical pass: one thread per (field, column).
-__global__ void k_blur_v(const MeField* __restrict__ mf, int nf, const float* __restrict__ src,
-                         float* __restrict__ dst, int r, int src_sel) {
+// Lines of a band: as many as fit, 0 when not even one does.
+inline int row_band(int n) {
+  return (int)std::min<size_t>(kRowBand, kBoxSmem / (sizeof(double) * row_stride(n)));
+}
+inline int col_band(int n) {
+  const size_t line = sizeof(double) * (n + 1);
+  return kBoxSmem / line >= kColBand ? kColBand : kBoxSmem / line >= 4 ? 4 : kBoxSmem / line >= 1;
+}
+
+// Vertical pass: one block per (field, 16-column band).
+__global__ void __launch_bounds__(kBoxThreads) k_blur_v(const MeField* __restrict__ mf, int nf,
+                                                        const float* __restrict__ src, float* dst,
+                                                        int r, int src_sel, int band) {
   const int f = blockIdx.y;
   if (f >= nf) return;
   const MeField m = mf[f];
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= m.w) return;
-  const int64_t sb = src_sel == 0 ? m.y_off : m.b_off;
-  const float* s = src + sb;
-  float* d = dst + m.t_off;
   const double norm = (double)(1.0f / (float)(2 * r + 1));
-  box_line(s + x, m.pitch, d + x, m.pitch, m.h, r, norm);
+  const float* s = src + (src_sel == 0 ? m.y_off : m.b_off);
+  if (band == 0) {
+    const int x = blockIdx.x * kBoxThreads + threadIdx.x;
+    if (x < m.w) box_line_long(s + x, dst + m.t_off + x, m.pitch, m.h, r, norm);
+    return;
+  }
+  const int x0 = blockIdx.x * band;
+  if (x0 >= m.w) return;
+  box_cols(s + x0, dst + m.t_off + x0, m.pitch, band, min(band, m.w - x0), m.h, r, norm);
 }
 
-// Horizontal pass: one warp per (field, 32-row band).
-__global__ void k_blur_h(const MeField* __restrict__ mf, int nf, const float* __restrict__ src,
-                         float* __restrict__ dst, int r) {
+// Horizontal pass: one block per (field, 8-row band).
+__global__ void __launch_bounds__(kBoxThreads) k_blur_h(const MeField* __restrict__ mf, int nf,
+                                                        const float* __restrict__ src, float* dst,
+                                                        int r, int band) {
   const int f = blockIdx.y;
   if (f >= nf) return;
   const MeField m = mf[f];
-  const int y0 = blockIdx.x * 32;
+  const double norm = (double)(1.0f / (float)(2 * r + 1));
+  const float* s = src + m.t_off;
+  float* d = dst + m.b_off;
+  if (band == 0) {
+    const int y = blockIdx.x * kBoxThreads + threadIdx.x;
+    if (y < m.h)
+      box_line_long(s + (int64_t)y * m.pitch, d + (int64_t)y * m.pitch, 1, m.w, r, norm);
+    return;
+  }
+  const int y0 = blockIdx.x * band;
   if (y0 >= m.h) return;
-  const double norm = (double)(1.0f / (float)(2 * r + 1));
-  box_rows_warp(src + m.t_off + (int64_t)y0 * m.pitch, dst + m.b_off + (int64_t)y0 * m.pitch,
-                m.pitch, min(32, m.h - y0), m.w, r, norm);
+  box_rows(s + (int64_t)y0 * m.pitch, d + (int64_t)y0 * m.pitch, m.pitch, min(band, m.h - y0), m.w,
+           r, norm);
 }
 
 // ---- Decimate (motion.cpp:59-78): 4 x 4 block mean ---------------------------
@@ -293,6 +218,9 @@ __device__ __forceinline__ float tile_ssd(const float* A, const float* B, int pi
 // centre-out candidate order (RangeFromCentre, motion.cpp:286-298) for a
 // symmetric range [-r, r]: 0, -1, 1, -2, 2, ...
 __device__ __forceinline__ int centre_out(int i) { return (i & 1) ? -((i + 1) >> 1) : (i >> 1); }
+__device__ __forceinline__ int centre_out_index(int d) {
+  return d == 0 ? 0 : (d > 0 ? 2 * d : -2 * d - 1);
+}
 
 // ---- coarse absolute pass on the 4x-decimated planes (motion.cpp:406-413) --
 __global__ void k_me_coarse(const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
@@ -337,70 +265,75 @@ __global__ void k_me_coarse(const MeField* __restrict__ mf, const MePair* __rest
   cdx[a.coarse_off * p + t] = bdx;
 }
 
-// The coarse pass with a warp per (pair, coarse tile) when the candidates
-// and tile rows fit (n^2 <= kCoarseWarpCands, ct <= kCoarseWarpRows): lanes
-// sum the candidates' SSD row by row in the reference's order, one lane
-// replays the visit from the per-row running sums (the zero vector, whose
-// cost needs the full sum, is never cut), as in k_me_refine_warp.
-constexpr int kCoarseWarpCands = 128;
-constexpr int kCoarseWarpRows = 16;
+// Candidates, tile rows and reach of k_me_coarse_tile; larger coarse tiles or
+// searches keep a thread per tile (k_me_coarse).
+constexpr int kCoarseCands = 128;
+constexpr int kCoarseRows = 16;
+constexpr int kCoarseReach = 5;  // (2 * 5 + 1)^2 <= kCoarseCands
 
-__global__ void k_me_coarse_warp(const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
-                                 int npairs, const float* __restrict__ dec, MeArgs a,
-                                 float* __restrict__ cdy, float* __restrict__ cdx) {
-  extern __shared__ float mc_part[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wpc = blockDim.x >> 5;
+// The coarse search of one tile by a block: the tile and the window its
+// candidates reach are staged in shared memory (clamped coordinates resolved
+// there), a thread runs one candidate's sum in the reference's order, keeping
+// the running sum after every row, and a warp replays the reference's visit
+// from those sums: kill = best * (1 / bias), the first row whose running sum
+// reaches it (a ballot over the rows) ends the candidate with that sum,
+// strict-less update. Every cost and decision is the per-thread kernel's. A
+// warp per tile reading global memory took 53 us on a PAL pair (latency of
+// three rounds of 64 dependent loads), this takes 8.
+__global__ void __launch_bounds__(kCoarseCands) k_me_coarse_tile(
+    const MeField* __restrict__ mf, const MePair* __restrict__ pairs, int npairs,
+    const float* __restrict__ dec, MeArgs a, float* __restrict__ cdy, float* __restrict__ cdx) {
+  constexpr int kWin = kCoarseRows + 2 * kCoarseReach;
+  __shared__ float sa[kCoarseRows * kCoarseRows], sb[kWin * (kWin + 1)];
+  __shared__ float part[kCoarseCands * (kCoarseRows + 1)];
   const int p = blockIdx.y;
-  if (p >= npairs) return;
   const MePair pr = pairs[p];
   const MeField mc = mf[pr.cur], mr = mf[pr.ref];
   const int hd = mc.h / 4, wd = mc.w / 4;
   const int ct = a.tile / 4 > 4 ? a.tile / 4 : 4;
   const int th = (hd + ct - 1) / ct, tw = (wd + ct - 1) / ct;
-  const int t = blockIdx.x * wpc + warp;
-  if (t >= th * tw) return;  // the whole warp; only warp-level sync below
+  const int t = blockIdx.x;
+  if (t >= th * tw) return;
   const int ty = t / tw, tx = t % tw;
   const int cs = (a.search + 3) / 4 > 1 ? (a.search + 3) / 4 : 1;
-  const int n = 2 * cs + 1;
-  const int ncand = n * n;
-  float* part = mc_part + (size_t)warp * kCoarseWarpCands * kCoarseWarpRows;
+  const int n = 2 * cs + 1, ncand = n * n;
   const float* A = dec + mc.d_off;
   const float* B = dec + mr.d_off;
-  const int y0 = ty * ct, y1 = min((ty + 1) * ct, hd);
-  const int x0 = tx * ct, x1 = min((tx + 1) * ct, wd);
-  const int rows = y1 - y0;
-  for (int c = lane; c < ncand; c += 32) {
-    const int sy = centre_out(c / n), sx = centre_out(c % n);
+  const int y0 = ty * ct, x0 = tx * ct;
+  const int rows = min(ct, hd - y0), cols = min(ct, wd - x0);
+  const int ww = cols + 2 * cs;
+  for (int i = threadIdx.x; i < rows * cols; i += kCoarseCands)
+    sa[i] = A[(int64_t)(y0 + i / cols) * mc.dpitch + x0 + i % cols];
+  for (int i = threadIdx.x; i < (rows + 2 * cs) * ww; i += kCoarseCands)
+    sb[i] = B[(int64_t)clampi(y0 - cs + i / ww, 0, hd - 1) * mc.dpitch +
+              clampi(x0 - cs + i % ww, 0, wd - 1)];
+  __syncthreads();
+  const int c = threadIdx.x;
+  if (c < ncand) {
+    const float* b = sb + (cs - centre_out(c / n)) * ww + cs - centre_out(c % n);
     float acc = 0.0f;
-    for (int y = y0; y < y1; ++y) {
-      const float* arow = A + (int64_t)y * mc.dpitch;
-      const float* brow = B + (int64_t)clampi(y - sy, 0, hd - 1) * mc.dpitch;
-      for (int x = x0; x < x1; ++x) {
-        const float diff = arow[x] - brow[clampi(x - sx, 0, wd - 1)];
+    for (int y = 0; y < rows; ++y) {
+#pragma unroll 4
+      for (int x = 0; x < cols; ++x) {
+        const float diff = sa[y * cols + x] - b[y * ww + x];
         acc += diff * diff;
       }
-      part[c * kCoarseWarpRows + (y - y0)] = acc;
+      part[c * (kCoarseRows + 1) + y] = acc;
     }
   }
-  __syncwarp();
-  if (lane != 0) return;
-  float best = __int_as_float(0x7f800000);
-  float bdy = 0.0f, bdx = 0.0f;
-  for (int c = 0; c < ncand; ++c) {
-    const int dy = centre_out(c / n), dx = centre_out(c % n);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  const float inf = __int_as_float(0x7f800000);
+  float best = inf, bdy = 0.0f, bdx = 0.0f;
+  for (int k = 0; k < ncand; ++k) {
+    const int dy = centre_out(k / n), dx = centre_out(k % n);
     const float bias = 1.0f + 0.02f * (float)(abs(dy) + abs(dx));
     const float inv_bias = 1.0f / bias;
-    const bool exact = dy == 0 && dx == 0;
-    const float kill = exact ? __int_as_float(0x7f800000) : best * inv_bias;
-    const float* pc = part + c * kCoarseWarpRows;
-    float se = pc[rows - 1];
-    for (int r = 0; r < rows; ++r) {
-      if (pc[r] >= kill) {
-        se = pc[r];
-        break;
-      }
-    }
+    const float kill = dy == 0 && dx == 0 ? inf : best * inv_bias;
+    const float* pc = part + k * (kCoarseRows + 1);
+    const unsigned hit = __ballot_sync(0xffffffffu, lane < rows && pc[lane] >= kill);
+    const float se = pc[hit ? __ffs(hit) - 1 : rows - 1];
     const float cost = se * bias;
     if (cost < best) {
       best = cost;
@@ -408,8 +341,10 @@ __global__ void k_me_coarse_warp(const MeField* __restrict__ mf, const MePair* _
       bdx = (float)dx;
     }
   }
-  cdy[a.coarse_off * p + t] = bdy;
-  cdx[a.coarse_off * p + t] = bdx;
+  if (lane == 0) {
+    cdy[a.coarse_off * p + t] = bdy;
+    cdx[a.coarse_off * p + t] = bdx;
+  }
 }
 
 // ---- full-res refinement, sub-pel fit, zero / margin rule (motion.cpp:415-473)
@@ -499,36 +434,45 @@ __global__ void k_me_refine(const MeField* __restrict__ mf, const MePair* __rest
   out_best[o] = best;
 }
 
-// The same refinement with a warp per (pair, tile), for tiles of up to
-// kRefineWarpTile rows. Lane l computes the SSD of refine candidates l and
-// l + 32 (visit order) row by row in the reference's order, without the
-// bail-out, keeping the running sum after every row in shared memory. The
-// warp then replays the reference's visit from those sums -- kill = best *
-// (1 / bias), the first row whose running sum reaches it (a ballot over the
-// rows) ends the candidate with that sum, strict-less update -- so every
-// cost, decision and vector is the per-thread kernel's; lanes 0-4 then take
-// the four CostAt sums and the zero-motion cost (full sums) at once.
+// The full-resolution refinement of one tile by a block of three warps: the
+// tile, the reference window that the +-3 candidates and their +-1 neighbours
+// reach and the unshifted reference tile are staged in shared memory. Thread
+// c runs the sum of one of the 81 shifts within +-4 of the base, thread 81
+// the zero-motion one, each in the reference's order; the inner 49 keep their
+// running sum after every row. The window's pitch is 9 modulo 32, so the
+// shifts of a warp fall into different banks. A warp then replays the
+// reference's visit as the coarse search does, and takes the four CostAt sums
+// and the zero-motion cost from the full sums -- the same sums in the same
+// order, so every cost, decision and vector is the per-thread kernel's. What
+// bounds it is one chained addition per pixel of the tile (4 cycles, 2 us for
+// 32 x 32); a warp per tile with its operands in global memory and the five
+// CostAt sums after the candidates took 187 us on a PAL pair, this takes 11.
 constexpr int kRefineCands = 49;  // RangeFromCentre(-3, 3)^2
-constexpr int kRefineWarpTile = 64;
+constexpr int kRefineTile = 64;
+constexpr int kRefineThreads = 96;
 
-__global__ void k_me_refine_warp(const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
-                                 int npairs, const float* __restrict__ blur, MeArgs a,
-                                 const float* __restrict__ cdy, const float* __restrict__ cdx,
-                                 float* __restrict__ out_mdy, float* __restrict__ out_mdx,
-                                 float* __restrict__ out_sdy, float* __restrict__ out_sdx,
-                                 float* __restrict__ out_best) {
+__host__ __device__ constexpr int refine_pitch(int cols) {
+  return (cols + 8 + 31 - 9) / 32 * 32 + 9;  // >= cols + 8, 9 modulo 32
+}
+inline size_t refine_smem(int tile) {
+  return sizeof(float) * (tile * tile + (size_t)(2 * tile + 8) * refine_pitch(tile) +
+                          kRefineCands * (tile + 1) + 82);
+}
+
+__global__ void __launch_bounds__(kRefineThreads) k_me_refine_tile(
+    const MeField* __restrict__ mf, const MePair* __restrict__ pairs, int npairs,
+    const float* __restrict__ blur, MeArgs a, const float* __restrict__ cdy,
+    const float* __restrict__ cdx, float* __restrict__ out_mdy, float* __restrict__ out_mdx,
+    float* __restrict__ out_sdy, float* __restrict__ out_sdx, float* __restrict__ out_best) {
   extern __shared__ float me_part[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wpc = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int p = blockIdx.y;
-  if (p >= npairs) return;
   const MePair pr = pairs[p];
   const MeField mc = mf[pr.cur], mr = mf[pr.ref];
   const int h = mc.h, w = mc.w, tile = a.tile;
   const int th = (h + tile - 1) / tile, tw = (w + tile - 1) / tile;
-  const int t = blockIdx.x * wpc + warp;
-  if (t >= th * tw) return;  // the whole warp; only warp-level sync below
-  float* part = me_part + (size_t)warp * kRefineCands * tile;
+  const int t = blockIdx.x;
+  if (t >= th * tw) return;
   const int ty = t / tw, tx = t % tw;
   const int hd = h / 4, wd = w / 4;
   const int ct = tile / 4 > 4 ? tile / 4 : 4;
@@ -540,39 +484,61 @@ __global__ void k_me_refine_warp(const MeField* __restrict__ mf, const MePair* _
   const float* B = blur + mr.b_off;
   const int y0 = ty * tile, y1 = min((ty + 1) * tile, h);
   const int x0 = tx * tile, x1 = min((tx + 1) * tile, w);
-  const int rows = y1 - y0;
+  const int rows = y1 - y0, cols = x1 - x0;
+  const int pitch = refine_pitch(tile);
+  float* sa = me_part;                      // rows x cols
+  float* sb = sa + tile * tile;             // (rows + 8) x pitch
+  float* s0 = sb + (tile + 8) * pitch;      // rows x pitch, unshifted
+  float* part = s0 + tile * pitch;          // kRefineCands x (tile + 1), in visit order
+  float* full = part + kRefineCands * (tile + 1);  // 81 shifts, then zero motion
   const float inf = __int_as_float(0x7f800000);
   const int rby = (int)lroundf(base_dy), rbx = (int)lroundf(base_dx);
-  for (int c = lane; c < kRefineCands; c += 32) {
-    const int sy = rby + centre_out(c / 7), sx = rbx + centre_out(c % 7);
+  for (int i = threadIdx.x; i < rows * cols; i += kRefineThreads) {
+    const int y = i / cols, x = i - y * cols;
+    sa[i] = A[(int64_t)(y0 + y) * mc.pitch + x0 + x];
+    s0[y * pitch + x] = B[(int64_t)(y0 + y) * mc.pitch + x0 + x];
+  }
+  for (int i = threadIdx.x; i < (rows + 8) * (cols + 8); i += kRefineThreads) {
+    const int y = i / (cols + 8), x = i - y * (cols + 8);
+    sb[y * pitch + x] = B[(int64_t)clampi(y0 - rby - 4 + y, 0, h - 1) * mc.pitch +
+                          clampi(x0 - rbx - 4 + x, 0, w - 1)];
+  }
+  __syncthreads();
+  const int c = threadIdx.x;
+  if (c < 82) {
+    const int cy = c / 9 - 4, cx = c % 9 - 4;  // shift of thread c < 81
+    const float* b = c < 81 ? sb + (4 - cy) * pitch + 4 - cx : s0;
+    const bool inner = c < 81 && abs(cy) <= 3 && abs(cx) <= 3;
+    float* pc = part + (inner ? centre_out_index(cy) * 7 + centre_out_index(cx) : 0) * (tile + 1);
     float acc = 0.0f;
-    for (int y = y0; y < y1; ++y) {
-      const float* arow = A + (int64_t)y * mc.pitch;
-      const float* brow = B + (int64_t)clampi(y - sy, 0, h - 1) * mc.pitch;
-      for (int x = x0; x < x1; ++x) {
-        const float diff = arow[x] - brow[clampi(x - sx, 0, w - 1)];
+    for (int y = 0; y < rows; ++y) {
+      const float* ar = sa + y * cols;
+      const float* br = b + y * pitch;
+#pragma unroll 8
+      for (int x = 0; x < cols; ++x) {
+        const float diff = ar[x] - br[x];
         acc += diff * diff;
       }
-      part[c * tile + (y - y0)] = acc;
+      if (inner) pc[y] = acc;
     }
+    full[c] = acc;
   }
-  __syncwarp();
-  // the reference's visit, the whole warp in step: for each candidate the
-  // first row whose running sum reaches kill is found by a ballot over the
-  // rows (lane r holds row r, r + 32), so every lane makes the same decisions
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
   float best = inf, mdy = 0.0f, mdx = 0.0f;
-  for (int c = 0; c < kRefineCands; ++c) {
-    const int dy = centre_out(c / 7), dx = centre_out(c % 7);
+  int bdy = 0, bdx = 0;
+  for (int k = 0; k < kRefineCands; ++k) {
+    const int dy = centre_out(k / 7), dx = centre_out(k % 7);
     const float bias = 1.0f + 0.02f * (float)(abs(dy) + abs(dx));
     const float inv_bias = 1.0f / bias;
     const float kill = best * inv_bias;
-    const float* pc = part + c * tile;
+    const float* pc = part + k * (tile + 1);
     float se = pc[rows - 1];
     for (int r0 = 0; r0 < rows; r0 += 32) {
-      const bool hit = r0 + lane < rows && pc[r0 + lane] >= kill;
-      const unsigned b = __ballot_sync(0xffffffffu, hit);
-      if (b) {
-        se = pc[r0 + __ffs(b) - 1];
+      const unsigned hit =
+          __ballot_sync(0xffffffffu, r0 + lane < rows && pc[r0 + lane] >= kill);
+      if (hit) {
+        se = pc[r0 + __ffs(hit) - 1];
         break;
       }
     }
@@ -581,25 +547,27 @@ __global__ void k_me_refine_warp(const MeField* __restrict__ mf, const MePair* _
       best = cost;
       mdy = base_dy + (float)dy;
       mdx = base_dx + (float)dx;
+      bdy = dy;
+      bdx = dx;
     }
   }
-  // CostAt at (+-1, 0), (0, +-1) and the zero-motion cost: full sums
-  const int iy = (int)lroundf(mdy), ix = (int)lroundf(mdx);
-  float v = 0.0f;
-  if (lane < 5) {
-    int sy = iy, sx = ix;
-    if (lane == 0) sy = (int)lroundf(mdy + -1.0f);
-    if (lane == 1) sy = (int)lroundf(mdy + 1.0f);
-    if (lane == 2) sx = (int)lroundf(mdx + -1.0f);
-    if (lane == 3) sx = (int)lroundf(mdx + 1.0f);
-    if (lane == 4) sy = sx = 0;
-    v = tile_ssd(A, B, mc.pitch, h, w, y0, y1, x0, x1, sy, sx, inf) * 1.0f;
+  // CostAt at (+-1, 0), (0, +-1) and the zero-motion cost: full sums. Where no
+  // cost is below infinity (non-finite planes) the visit keeps no candidate and
+  // CostAt looks around zero motion.
+  const float cost0 = full[81] * 1.0f;
+  float cym, cyp, cxm, cxp;
+  if (best < inf) {
+    const float* fc = full + (bdy + 4) * 9 + bdx + 4;
+    cym = fc[-9] * 1.0f;
+    cyp = fc[9] * 1.0f;
+    cxm = fc[-1] * 1.0f;
+    cxp = fc[1] * 1.0f;
+  } else {
+    cym = tile_ssd(A, B, mc.pitch, h, w, y0, y1, x0, x1, -1, 0, inf) * 1.0f;
+    cyp = tile_ssd(A, B, mc.pitch, h, w, y0, y1, x0, x1, 1, 0, inf) * 1.0f;
+    cxm = tile_ssd(A, B, mc.pitch, h, w, y0, y1, x0, x1, 0, -1, inf) * 1.0f;
+    cxp = tile_ssd(A, B, mc.pitch, h, w, y0, y1, x0, x1, 0, 1, inf) * 1.0f;
   }
-  const float cym = __shfl_sync(0xffffffffu, v, 0);
-  const float cyp = __shfl_sync(0xffffffffu, v, 1);
-  const float cxm = __shfl_sync(0xffffffffu, v, 2);
-  const float cxp = __shfl_sync(0xffffffffu, v, 3);
-  const float cost0 = __shfl_sync(0xffffffffu, v, 4);
   if (lane != 0) return;
   auto parabolic = [](float cm, float c0, float cp) {
     const float den = cm - 2.0f * c0 + cp;
@@ -630,72 +598,107 @@ __global__ void k_me_refine_warp(const MeField* __restrict__ mf, const MePair* _
   out_best[o] = best;
 }
 
-// ---- MotionConfidence (motion.cpp:321-387) + final vectors. One CTA per pair.
-__global__ void __launch_bounds__(256) k_me_confidence(const MeField* __restrict__ mf,
-                                                       const MePair* __restrict__ pairs,
-                                                       int npairs, const float* __restrict__ blur,
-                                                       MeArgs a, const float* __restrict__ mdy,
+// ---- MotionConfidence (motion.cpp:321-387) + final vectors ------------------
+// (1) A tile's mean, variance and residual ratio: a warp per tile brings the
+// tile to shared memory kConfChunk pixels at a time (row by row, coalesced)
+// and one lane adds them in the reference's order; conf0 and the ratio go to
+// out_conf / out_dy for (2). The two chained additions per pixel bound it (3
+// us for 32 x 32); one thread per tile of one block per pair, with the medians
+// behind it, took 190 us on a PAL pair, (1) and (2) take 16.
+constexpr int kConfChunk = 1024;
+constexpr int kConfWarps = 8;
+__global__ void __launch_bounds__(32 * kConfWarps) k_me_tile_stats(
+    const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
+    const float* __restrict__ blur, MeArgs a, const float* __restrict__ bestv,
+    float* __restrict__ out_ratio, float* __restrict__ out_conf0) {
+  __shared__ float px[kConfWarps][kConfChunk];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p = blockIdx.y;
+  const MeField mc = mf[pairs[p].cur];
+  const int h = mc.h, w = mc.w, tile = a.tile;
+  const int th = (h + tile - 1) / tile, tw = (w + tile - 1) / tile;
+  const int t = blockIdx.x * kConfWarps + warp;
+  if (t >= th * tw) return;  // the whole warp; only warp-level sync below
+  // rows/cols mapped by min(y / tile, th - 1)
+  const int y0 = t / tw * tile, x0 = t % tw * tile;
+  const int cols = min(tile, w - x0), n = min(tile, h - y0) * cols;
+  const float* A = blur + mc.b_off + (int64_t)y0 * mc.pitch + x0;
+  float* v = px[warp];
+  float sum = 0.0f, sum2 = 0.0f;
+  for (int i0 = 0; i0 < n; i0 += kConfChunk) {
+    const int m = min(kConfChunk, n - i0);
+#pragma unroll 8
+    for (int i = lane; i < m; i += 32)
+      v[i] = A[(int64_t)((i0 + i) / cols) * mc.pitch + (i0 + i) % cols];
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll 16
+      for (int i = 0; i < m; ++i) {
+        const float x = v[i];
+        sum += x;
+        sum2 += x * x;
+      }
+    }
+    __syncwarp();
+  }
+  if (lane != 0) return;
+  // the reference counts pixels in float: exact below 2^24, and a tile has fewer
+  const float np = (float)n;
+  const float norm = 1.0f / fmaxf(1.0f, np);
+  const float tmean = sum * norm;
+  const float tvar = sum2 * norm - tmean * tmean;
+  const int o = a.tiles_off * p + t;
+  const float best = bestv[o];
+  const float energy = (tvar + 1.0f) * fmaxf(1.0f, np);
+  out_conf0[o] = fminf(fmaxf(1.0f - best / energy, 0.0f), 1.0f);
+  out_ratio[o] = best / fmaxf(1.0f, np);
+}
+
+// (2) The median ratio and the final confidences and vectors, one block per
+// pair; the two middle ratios by counting ranks (a few hundred tiles), by
+// radix selection past kRankTiles.
+constexpr int kRankTiles = 1024;
+__global__ void __launch_bounds__(256) k_me_confidence(const MePair* __restrict__ pairs, MeArgs a,
+                                                       int nt, const float* __restrict__ mdy,
                                                        const float* __restrict__ mdx,
                                                        const float* __restrict__ sdy,
                                                        const float* __restrict__ sdx,
-                                                       const float* __restrict__ bestv,
                                                        float* __restrict__ out_dy,
                                                        float* __restrict__ out_dx,
                                                        float* __restrict__ out_conf) {
-  extern __shared__ float me_sm[];
+  extern __shared__ float ratios[];  // nt
   __shared__ unsigned hist[256];
   __shared__ unsigned bc[2];
-  const int p = blockIdx.x;
-  const MePair pr = pairs[p];
-  const MeField mc = mf[pr.cur];
-  const int h = mc.h, w = mc.w, tile = a.tile;
-  const int th = (h + tile - 1) / tile, tw = (w + tile - 1) / tile;
-  const int nt = th * tw;
-  float* ratios = me_sm;         // nt
-  float* conf0 = me_sm + nt;     // nt
-  const float* A = blur + mc.b_off;
-  const int o = a.tiles_off * p;
-  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-    const int ty = t / tw, tx = t % tw;
-    // pixels of this tile: rows/cols mapped by min(y / tile, th - 1)
-    const int y0 = ty * tile, y1 = (ty == th - 1) ? h : (ty + 1) * tile;
-    const int x0 = tx * tile, x1 = (tx == tw - 1) ? w : (tx + 1) * tile;
-    float sum = 0.0f, sum2 = 0.0f, np = 0.0f;
-    for (int y = y0; y < y1; ++y) {
-      const float* arow = A + (int64_t)y * mc.pitch;
-      // eight samples' loads ahead of their additions, which stay in x order
-      for (int xb = x0; xb < x1; xb += 8) {
-        float v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = arow[xb + q < x1 ? xb + q : x1 - 1];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (xb + q < x1) {
-            sum += v[q];
-            sum2 += v[q] * v[q];
-            np += 1.0f;
-          }
-      }
-    }
-    const float norm = 1.0f / fmaxf(1.0f, np);
-    const float tmean = sum * norm;
-    const float tvar = sum2 * norm - tmean * tmean;
-    const float best = bestv[o + t];
-    const float energy = (tvar + 1.0f) * fmaxf(1.0f, np);
-    conf0[t] = fminf(fmaxf(1.0f - best / energy, 0.0f), 1.0f);
-    ratios[t] = best / fmaxf(1.0f, np);
-  }
+  __shared__ float mid[2];
+  const int o = a.tiles_off * blockIdx.x;
+  for (int t = threadIdx.x; t < nt; t += blockDim.x) ratios[t] = out_dy[o + t];
   __syncthreads();
   // Median (motion.cpp:80-91): nth_element at n/2, averaged with the (n/2-1)-th for even n
   const int k = nt / 2;
-  float med = block_select_kth(ratios, nt, k, hist, bc);
-  if (nt % 2 == 0) {
-    const float lo = block_select_kth(ratios, nt, k - 1, hist, bc);
-    med = 0.5f * (med + lo);
+  float med, lo;
+  if (nt <= kRankTiles) {
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+      const uint32_t key = float_key(ratios[t]);
+      int less = 0, eq = 0;
+      for (int u = 0; u < nt; ++u) {
+        const uint32_t ku = float_key(ratios[u]);
+        less += ku < key;
+        eq += ku == key;
+      }
+      if (less <= k && k < less + eq) mid[0] = ratios[t];
+      if (less <= k - 1 && k - 1 < less + eq) mid[1] = ratios[t];
+    }
+    __syncthreads();
+    med = mid[0];
+    lo = nt % 2 == 0 ? mid[1] : 0.0f;
+  } else {
+    med = block_select_kth(ratios, nt, k, hist, bc);
+    lo = nt % 2 == 0 ? block_select_kth(ratios, nt, k - 1, hist, bc) : 0.0f;
   }
+  if (nt % 2 == 0) med = 0.5f * (med + lo);
   for (int t = threadIdx.x; t < nt; t += blockDim.x) {
     const float excess = fmaxf(0.0f, ratios[t] - med);
-    float c = conf0[t];
+    float c = out_conf[o + t];
     c *= (med + 1.0f) / (med + 1.0f + excess);
     c *= 6.0f / (6.0f + med);
     out_conf[o + t] = c;
@@ -704,48 +707,46 @@ __global__ void __launch_bounds__(256) k_me_confidence(const MeField* __restrict
   }
 }
 
+static void field_blur(const MeField* d_fields, int nf, int max_h, int max_w, const MeBuffers& b,
+                       cudaStream_t st);
+static PerDeviceOnce refine_once;
+
 void launch_motion_blur(const MeField* d_fields, int nf, int max_h, int max_w, const MeBuffers& b,
                         cudaStream_t st) {
   if (nf <= 0) return;
-  k_blur_v<<<dim3((max_w + kBoxThreads - 1) / kBoxThreads, nf), kBoxThreads, 0, st>>>(
-      d_fields, nf, b.luma, b.tmp, 2, 0);
-  k_blur_h<<<dim3((max_h + 31) / 32, nf), 32, 0, st>>>(d_fields, nf, b.tmp, b.blur, 2);
+  field_blur(d_fields, nf, max_h, max_w, b, st);
 }
 
 void launch_motion(const MeField* d_fields, int nf, int max_h, int max_w, const MePair* d_pairs,
                    int npairs, const MeArgs& a, const MeBuffers& b, cudaStream_t st) {
   if (nf <= 0 || npairs <= 0) return;
-  const int r = 2;
   // blur every field's luma (A = blur(y_cur), B = blur(y_ref) share per field)
-  k_blur_v<<<dim3((max_w + kBoxThreads - 1) / kBoxThreads, nf), kBoxThreads, 0, st>>>(
-      d_fields, nf, b.luma, b.tmp, r, 0);
-  k_blur_h<<<dim3((max_h + 31) / 32, nf), 32, 0, st>>>(d_fields, nf, b.tmp, b.blur, r);
+  field_blur(d_fields, nf, max_h, max_w, b, st);
   k_decimate<<<dim3(((max_h / 4) * (max_w / 4) + 255) / 256, nf), 256, 0, st>>>(d_fields, nf, b.blur, b.dec);
   const int ct = a.tile / 4 > 4 ? a.tile / 4 : 4;
   const int cth = ((max_h / 4) + ct - 1) / ct, ctw = ((max_w / 4) + ct - 1) / ct;
   const int cn = 2 * ((a.search + 3) / 4 > 1 ? (a.search + 3) / 4 : 1) + 1;
-  if (cn * cn <= kCoarseWarpCands && ct <= kCoarseWarpRows) {
-    const int wpc = 4;
-    const int csmem = wpc * kCoarseWarpCands * kCoarseWarpRows * (int)sizeof(float);
-    k_me_coarse_warp<<<dim3((cth * ctw + wpc - 1) / wpc, npairs), 32 * wpc, csmem, st>>>(
+  if (cn * cn <= kCoarseCands && ct <= kCoarseRows) {
+    k_me_coarse_tile<<<dim3(cth * ctw, npairs), kCoarseCands, 0, st>>>(
         d_fields, d_pairs, npairs, b.dec, a, b.cdy, b.cdx);
   } else {
     k_me_coarse<<<dim3((cth * ctw + 63) / 64, npairs), 64, 0, st>>>(d_fields, d_pairs, npairs,
                                                                  b.dec, a, b.cdy, b.cdx);
   }
   const int th = (max_h + a.tile - 1) / a.tile, tw = (max_w + a.tile - 1) / a.tile;
-  if (a.tile <= kRefineWarpTile) {
-    const int wpc = a.tile <= 32 ? 4 : 2;
-    const int rsmem = wpc * kRefineCands * a.tile * (int)sizeof(float);
-    k_me_refine_warp<<<dim3((th * tw + wpc - 1) / wpc, npairs), 32 * wpc, rsmem, st>>>(
+  if (a.tile <= kRefineTile) {
+    refine_once([] {
+      cudaFuncSetAttribute(k_me_refine_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)refine_smem(kRefineTile));
+    });
+    k_me_refine_tile<<<dim3(th * tw, npairs), kRefineThreads, refine_smem(a.tile), st>>>(
         d_fields, d_pairs, npairs, b.blur, a, b.cdy, b.cdx, b.mdy, b.mdx, b.sdy, b.sdx, b.best);
   } else {
     k_me_refine<<<dim3((th * tw + 63) / 64, npairs), 64, 0, st>>>(
         d_fields, d_pairs, npairs, b.blur, a, b.cdy, b.cdx, b.mdy, b.mdx, b.sdy, b.sdx, b.best);
   }
-  const int smem = 2 * th * tw * (int)sizeof(float);
-  k_me_confidence<<<npairs, 256, smem, st>>>(d_fields, d_pairs, npairs, b.blur, a, b.mdy, b.mdx,
-                                             b.sdy, b.sdx, b.best, b.dy, b.dx, b.conf);
+  launch_me_confidence(d_fields, d_pairs, npairs, max_h, max_w, a, b.blur, b.mdy, b.mdx, b.sdy,
+                       b.sdx, b.best, b.dy, b.dx, b.conf, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -783,61 +784,39 @@ __device__ __forceinline__ int quant_luma(float y) {
   return (int)fminf(fmaxf(rintf(t), 0.0f), 65535.0f);
 }
 
-// Vertical 5-row window sums of the quantised luma (zero outside the field).
-// One thread per (field, column).
-__global__ void k_sad_vsum(const MeField* __restrict__ mf, int nf, const float* __restrict__ luma,
-                           int* __restrict__ vsum) {
-  const int f = blockIdx.y;
-  const MeField m = mf[f];
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= m.w) return;
+// The quantised luma's 5 x 5 box (zero outside the field), rounded: integer
+// sums, so any order is exact. A block takes a 64 x 16 tile with its border
+// into shared memory, sums columns, then rows. One pass over the plane in
+// place of a running sum per column and then per row (two 760 x 242 planes:
+// 358 -> 6 us).
+constexpr int kQbX = 64, kQbY = 16;
+__global__ void __launch_bounds__(256) k_sad_blur(const MeField* __restrict__ mf,
+                                                  const float* __restrict__ luma,
+                                                  int* __restrict__ qblur) {
+  __shared__ int q[kQbY + 4][kQbX + 4];
+  __shared__ int v[kQbY][kQbX + 4];
+  const MeField m = mf[blockIdx.z];
+  const int x0 = blockIdx.x * kQbX, y0 = blockIdx.y * kQbY;
+  if (x0 >= m.w || y0 >= m.h) return;
   const float* Y = luma + m.y_off;
-  int* V = vsum + m.t_off;
-  int ring[5] = {0, 0, 0, 0, 0};
-  int acc = 0;
-  // rows y - 2 .. y + 2; prime with rows 0 .. 1
-  for (int y = 0; y < 2 && y < m.h; ++y) {
-    ring[y] = quant_luma(Y[(int64_t)y * m.pitch + x]);
-    acc += ring[y];
+  for (int i = threadIdx.x; i < (kQbY + 4) * (kQbX + 4); i += 256) {
+    const int r = i / (kQbX + 4), c = i % (kQbX + 4), y = y0 + r - 2, x = x0 + c - 2;
+    q[r][c] = y >= 0 && y < m.h && x >= 0 && x < m.w ? quant_luma(Y[(int64_t)y * m.pitch + x]) : 0;
   }
-  for (int y = 0; y < m.h; ++y) {
-    const int yn = y + 2;
-    if (yn < m.h) {
-      const int q = quant_luma(Y[(int64_t)yn * m.pitch + x]);
-      acc += q;
-      ring[yn % 5] = q;
-    }
-    V[(int64_t)y * m.pitch + x] = acc;
-    const int yo = y - 2;
-    if (yo >= 0) {
-      acc -= ring[yo % 5];
-      ring[yo % 5] = 0;
-    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kQbY * (kQbX + 4); i += 256) {
+    const int r = i / (kQbX + 4), c = i % (kQbX + 4);
+    v[r][c] = q[r][c] + q[r + 1][c] + q[r + 2][c] + q[r + 3][c] + q[r + 4][c];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kQbY * kQbX; i += 256) {
+    const int r = i / kQbX, c = i % kQbX, y = y0 + r, x = x0 + c;
+    if (y < m.h && x < m.w)
+      qblur[m.b_off + (int64_t)y * m.pitch + x] =
+          (v[r][c] + v[r][c + 1] + v[r][c + 2] + v[r][c + 3] + v[r][c + 4] + 12) / 25;
   }
 }
 
-// Horizontal 5-column sums of vsum, rounded division by 25. One thread per
-// (field, row).
-__global__ void k_sad_hsum(const MeField* __restrict__ mf, int nf, const int* __restrict__ vsum,
-                           int* __restrict__ qblur) {
-  const int f = blockIdx.y;
-  const MeField m = mf[f];
-  const int y = blockIdx.x * blockDim.x + threadIdx.x;
-  if (y >= m.h) return;
-  const int* V = vsum + m.t_off + (int64_t)y * m.pitch;
-  int* Q = qblur + m.b_off + (int64_t)y * m.pitch;
-  int acc = 0;
-  for (int x = 0; x < 2 && x < m.w; ++x) acc += V[x];
-  for (int x = 0; x < m.w; ++x) {
-    if (x + 2 < m.w) acc += V[x + 2];
-    Q[x] = (acc + 12) / 25;
-    if (x - 2 >= 0) acc -= V[x - 2];
-  }
-}
-
-__device__ __forceinline__ int centre_out_index(int d) {
-  return d == 0 ? 0 : (d > 0 ? 2 * d : -2 * d - 1);
-}
 
 // SAD (or SSD) over the tile of source offset (dy, dx), one warp (lanes over pixels).
 __device__ __forceinline__ unsigned long long warp_tile_cost(const int* As, const int* Bs, int b,
@@ -1226,8 +1205,8 @@ void launch_motion_sad(const MeField* d_fields, int nf, int max_h, int max_w,
                        const MePair* d_pairs, int npairs, const SadArgs& a, const SadBuffers& b,
                        cudaStream_t st) {
   if (nf <= 0 || npairs <= 0) return;
-  k_sad_vsum<<<dim3((max_w + 127) / 128, nf), 128, 0, st>>>(d_fields, nf, b.luma, b.vsum);
-  k_sad_hsum<<<dim3((max_h + 127) / 128, nf), 128, 0, st>>>(d_fields, nf, b.vsum, b.qblur);
+  k_sad_blur<<<dim3((max_w + kQbX - 1) / kQbX, (max_h + kQbY - 1) / kQbY, nf), 256, 0, st>>>(
+      d_fields, b.luma, b.qblur);
   const int th = (max_h + a.block - 1) / a.block, tw = (max_w + a.block - 1) / a.block;
   const int ww = a.block + 2 * (a.range + 1);
   const int smem = sad_smem_ints(a.block, ww) * (int)sizeof(int);
@@ -1386,34 +1365,69 @@ __global__ void k_conf_pixels_nearest(const MeField* __restrict__ mf, const MePa
   out[pix_off[p] + (int64_t)y * mc.pitch + x] = c * c;
 }
 
-// BoxBlur radius r over per-pair planes (same prefix-sum arithmetic as the
-// luma blur); in place through a scratch plane.
-__global__ void k_pair_blur_v(const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
-                              int npairs, const float* __restrict__ src, float* __restrict__ dst,
-                              const int64_t* __restrict__ pix_off, int r) {
+// BoxBlur radius r over per-pair planes (the luma blur's arithmetic), and over
+// several channels `chan` floats apart: columns, then rows.
+__global__ void __launch_bounds__(kBoxThreads) k_pair_blur_v(
+    const MeField* __restrict__ mf, const MePair* __restrict__ pairs, int npairs, const float* src,
+    float* dst, const int64_t* __restrict__ pix_off, int64_t chan, int r, int band) {
   const int p = blockIdx.y;
   if (p >= npairs) return;
   const MeField m = mf[pairs[p].cur];
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= m.w) return;
-  const float* s = src + pix_off[p];
-  float* d = dst + pix_off[p];
-  const double norm = (double)(1.0f / (float)(2 * r + 1));
-  box_line(s + x, m.pitch, d + x, m.pitch, m.h, r, norm);
+  const int x0 = blockIdx.x * band;
+  if (x0 >= m.w) return;
+  const int64_t o = pix_off[p] + blockIdx.z * chan + x0;
+  box_cols(src + o, dst + o, m.pitch, band, min(band, m.w - x0), m.h, r,
+           (double)(1.0f / (float)(2 * r + 1)));
 }
 
-// one warp per (pair, 32-row band)
-__global__ void k_pair_blur_h(const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
-                              int npairs, const float* __restrict__ src, float* __restrict__ dst,
-                              const int64_t* __restrict__ pix_off, int r) {
+__global__ void __launch_bounds__(kBoxThreads) k_pair_blur_h(
+    const MeField* __restrict__ mf, const MePair* __restrict__ pairs, int npairs, float* plane,
+    const int64_t* __restrict__ pix_off, int64_t chan, int r, int band) {
   const int p = blockIdx.y;
   if (p >= npairs) return;
   const MeField m = mf[pairs[p].cur];
-  const int y0 = blockIdx.x * 32;
+  const int y0 = blockIdx.x * band;
   if (y0 >= m.h) return;
-  const double norm = (double)(1.0f / (float)(2 * r + 1));
-  box_rows_warp(src + pix_off[p] + (int64_t)y0 * m.pitch, dst + pix_off[p] + (int64_t)y0 * m.pitch,
-                m.pitch, min(32, m.h - y0), m.w, r, norm);
+  float* d = plane + pix_off[p] + blockIdx.z * chan + (int64_t)y0 * m.pitch;
+  box_rows(d, d, m.pitch, min(band, m.h - y0), m.w, r, (double)(1.0f / (float)(2 * r + 1)));
+}
+
+static PerDeviceOnce box_once;
+
+static void configure_box() {
+  box_once([] {
+    cudaFuncSetAttribute(k_blur_v, cudaFuncAttributeMaxDynamicSharedMemorySize, kBoxSmem);
+    cudaFuncSetAttribute(k_blur_h, cudaFuncAttributeMaxDynamicSharedMemorySize, kBoxSmem);
+    cudaFuncSetAttribute(k_pair_blur_v, cudaFuncAttributeMaxDynamicSharedMemorySize, kBoxSmem);
+    cudaFuncSetAttribute(k_pair_blur_h, cudaFuncAttributeMaxDynamicSharedMemorySize, kBoxSmem);
+  });
+}
+
+// The luma planes' blur (tmp, then blur).
+static void field_blur(const MeField* d_fields, int nf, int max_h, int max_w, const MeBuffers& b,
+                       cudaStream_t st) {
+  configure_box();
+  const int cb = col_band(max_h), rb = row_band(max_w);
+  const int cl = cb ? cb : kBoxThreads, rl = rb ? rb : kBoxThreads;  // lines per block
+  k_blur_v<<<dim3((max_w + cl - 1) / cl, nf), kBoxThreads, sizeof(double) * cb * (max_h + 1), st>>>(
+      d_fields, nf, b.luma, b.tmp, 2, 0, cb);
+  k_blur_h<<<dim3((max_h + rl - 1) / rl, nf), kBoxThreads,
+             sizeof(double) * rb * row_stride(max_w), st>>>(d_fields, nf, b.tmp, b.blur, 2, rb);
+}
+
+// `chans` channels of the pairs' planes (fields of a window: every line fits
+// shared memory): src -> dst, src and dst may be the same.
+static void pair_blur(const MeField* d_fields, const MePair* d_pairs, int npairs, int max_h,
+                      int max_w, const float* src, float* dst, const int64_t* pix_off, int chans,
+                      int64_t chan, int r, cudaStream_t st) {
+  configure_box();
+  const int cb = col_band(max_h), rb = row_band(max_w);
+  k_pair_blur_v<<<dim3((max_w + cb - 1) / cb, npairs, chans), kBoxThreads,
+                  sizeof(double) * cb * (max_h + 1), st>>>(d_fields, d_pairs, npairs, src, dst,
+                                                           pix_off, chan, r, cb);
+  k_pair_blur_h<<<dim3((max_h + rb - 1) / rb, npairs, chans), kBoxThreads,
+                  sizeof(double) * rb * row_stride(max_w), st>>>(d_fields, d_pairs, npairs, dst,
+                                                                 pix_off, chan, r, rb);
 }
 
 // ---------------------------------------------------------------------------
@@ -1498,65 +1512,42 @@ __global__ void k_traj_snap(const MeField* __restrict__ mf, const MePair* __rest
   }
 }
 
-// Fast-mode prediction (sequence.cpp:714-763) + VerifyMotion (motion.cpp:490-530).
-// Sum of squared differences over one tile with no bail-out (a lone
-// candidate: BmPass's kill stays infinite), rows in order and each row in
-// order -- the reference's float additions -- with each row's samples
-// loaded ahead of its additions.
-__device__ __forceinline__ float tile_ssd_full(const float* A, const float* B, int pitch, int h,
-                                               int w, int ty0, int ty1, int tx0, int tx1, int sy,
-                                               int sx) {
-  float acc = 0.0f;
-  for (int y = ty0; y < ty1; ++y) {
-    const float* arow = A + (int64_t)y * pitch;
-    const float* brow = B + (int64_t)clampi(y - sy, 0, h - 1) * pitch;
-    int x = tx0;
-    for (; x + 8 <= tx1; x += 8) {
-      float d[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) d[k] = arow[x + k] - brow[clampi(x + k - sx, 0, w - 1)];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc += d[k] * d[k];
-    }
-    for (; x < tx1; ++x) {
-      const float diff = arow[x] - brow[clampi(x - sx, 0, w - 1)];
-      acc += diff * diff;
-    }
-  }
-  return acc;
-}
-
 // VerifyMotion (motion.cpp:490-530) of pair base + i: one SSD at the rounded
 // prediction, one at zero, the prediction kept where it is strictly better.
 // The prediction is the trajectory median over the searched pairs of its
 // group (sequence.cpp:714-763), or, with pred_dy / pred_dx given, the
-// caller's per-tile vectors. Two adjacent threads per tile: the even one
-// evaluates the prediction, the odd one zero.
-__global__ void k_traj_verify(const MeField* __restrict__ mf, const MePair* __restrict__ pairs,
-                              int base, int npred, const int* __restrict__ grp,
-                              const TrajGroup* __restrict__ searched,
-                              const TrajPair* __restrict__ tp, const float* __restrict__ blur,
-                              MeArgs a, const float* __restrict__ dy_in,
-                              const float* __restrict__ dx_in, const float* __restrict__ pred_dy,
-                              const float* __restrict__ pred_dx, float* __restrict__ out_mdy,
-                              float* __restrict__ out_mdx, float* __restrict__ out_sdy,
-                              float* __restrict__ out_sdx, float* __restrict__ out_best) {
+// caller's per-tile vectors.
+//
+// A warp per tile: the squared differences of the prediction and of zero
+// motion are formed by all lanes into shared memory, kVerifyChunk pixels at a
+// time, and two lanes add them in the reference's order (4 cycles a pixel). A
+// thread per sum reading global memory took 95 us for 5 NTSC pairs, this 12.
+constexpr int kVerifyChunk = 1024;
+constexpr int kVerifyWarps = 4;
+__global__ void __launch_bounds__(32 * kVerifyWarps) k_traj_verify(
+    const MeField* __restrict__ mf, const MePair* __restrict__ pairs, int base, int npred,
+    const int* __restrict__ grp, const TrajGroup* __restrict__ searched,
+    const TrajPair* __restrict__ tp, const float* __restrict__ blur, MeArgs a,
+    const float* __restrict__ dy_in, const float* __restrict__ dx_in,
+    const float* __restrict__ pred_dy, const float* __restrict__ pred_dx,
+    float* __restrict__ out_mdy, float* __restrict__ out_mdx, float* __restrict__ out_sdy,
+    float* __restrict__ out_sdx, float* __restrict__ out_best) {
+  __shared__ float sq[kVerifyWarps][2][kVerifyChunk];
   const int i = blockIdx.y;
-  if (i >= npred) return;  // uniform per block
   const int p = base + i;
   const MePair pr = pairs[p];
   const MeField mc = mf[pr.cur], mr = mf[pr.ref];
   const int h = mc.h, w = mc.w, tile = a.tile;
   const int th = (h + tile - 1) / tile, tw = (w + tile - 1) / tile;
-  const int tt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = tt >> 1, cand = tt & 1;
-  const bool valid = t < th * tw;
-  float pdy = 0.0f, pdx = 0.0f, ssd = 0.0f;
-  if (valid) {
-    if (pred_dy) {
-      pdy = pred_dy[a.tiles_off * i + t];
-      pdx = pred_dx[a.tiles_off * i + t];
-    } else {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = blockIdx.x * kVerifyWarps + warp;
+  if (t >= th * tw) return;  // the whole warp; only warp-level sync below
+  float pdy = 0.0f, pdx = 0.0f;
+  if (pred_dy) {
+    pdy = pred_dy[a.tiles_off * i + t];
+    pdx = pred_dx[a.tiles_off * i + t];
+  } else {
+    if (lane == 0) {
       const TrajGroup S = searched[grp[i]];
       float sy[kTrajMaxPairs], sx[kTrajMaxPairs];
       for (int k = 0; k < S.count; ++k) {
@@ -1572,14 +1563,39 @@ __global__ void k_traj_verify(const MeField* __restrict__ mf, const MePair* __re
       pdy = (float)me.offset * vym0 + me.parity_shift;
       pdx = (float)me.offset * vxm0;
     }
-    const int iy = cand == 0 ? (int)lroundf(pdy) : 0, ix = cand == 0 ? (int)lroundf(pdx) : 0;
-    const int y0 = (t / tw) * tile, y1 = min(y0 + tile, h);
-    const int x0 = (t % tw) * tile, x1 = min(x0 + tile, w);
-    ssd = tile_ssd_full(blur + mc.b_off, blur + mr.b_off, mc.pitch, h, w, y0, y1, x0, x1, iy, ix);
+    pdy = __shfl_sync(0xffffffffu, pdy, 0);
+    pdx = __shfl_sync(0xffffffffu, pdx, 0);
   }
-  const float zero = __shfl_down_sync(0xffffffffu, ssd, 1);
-  if (!valid || cand != 0) return;
-  const float pred = ssd;
+  const int iy = (int)lroundf(pdy), ix = (int)lroundf(pdx);
+  const int y0 = t / tw * tile, x0 = t % tw * tile;
+  const int cols = min(tile, w - x0), n = min(tile, h - y0) * cols;
+  const float* A = blur + mc.b_off;
+  const float* B = blur + mr.b_off;
+  float* s0 = sq[warp][0];
+  float* s1 = sq[warp][1];
+  float acc = 0.0f;
+  for (int c0 = 0; c0 < n; c0 += kVerifyChunk) {
+    const int m = min(kVerifyChunk, n - c0);
+#pragma unroll 4
+    for (int k = lane; k < m; k += 32) {
+      const int y = y0 + (c0 + k) / cols, x = x0 + (c0 + k) % cols;
+      const float v = A[(int64_t)y * mc.pitch + x];
+      const float dp = v - B[(int64_t)clampi(y - iy, 0, h - 1) * mc.pitch + clampi(x - ix, 0, w - 1)];
+      const float dz = v - B[(int64_t)y * mc.pitch + x];
+      s0[k] = dp * dp;
+      s1[k] = dz * dz;
+    }
+    __syncwarp();
+    if (lane < 2) {
+      const float* v = lane == 0 ? s0 : s1;
+#pragma unroll 16
+      for (int k = 0; k < m; ++k) acc += v[k];
+    }
+    __syncwarp();
+  }
+  const float zero = __shfl_sync(0xffffffffu, acc, 1);
+  if (lane != 0) return;
+  const float pred = acc;
   const int o = a.tiles_off * p + t;
   if (zero <= pred) {
     out_mdy[o] = 0.0f;
@@ -1696,14 +1712,7 @@ void launch_vectors(const MeField* d_fields, const MePair* d_pairs, int npairs, 
   } else {
     k_conf_pixels_nearest<<<dim3((max_w + 127) / 128, max_h, npairs), 128, 0, st>>>(
         d_fields, d_pairs, npairs, a, v.conf, v.conf_tmp, v.pix_off);
-    k_pair_blur_v<<<dim3((max_w + kBoxThreads - 1) / kBoxThreads, npairs), kBoxThreads, 0,
-                    st>>>(d_fields, d_pairs, npairs,
-                                                                     v.conf_tmp, v.conf_px,
-                                                                     v.pix_off, 8);
-    k_pair_blur_h<<<dim3((max_h + 31) / 32, npairs), 32, 0, st>>>(d_fields, d_pairs, npairs,
-                                                                  v.conf_px, v.conf_tmp,
-                                                                  v.pix_off, 8);
-    cudaMemcpyAsync(v.conf_px, v.conf_tmp, v.conf_bytes, cudaMemcpyDeviceToDevice, st);
+    pair_blur(d_fields, d_pairs, npairs, max_h, max_w, v.conf_tmp, v.conf_px, v.pix_off, 1, 0, 8, st);
   }
 }
 
@@ -1724,7 +1733,7 @@ void launch_traj_verify(const MeField* d_fields, const MePair* d_pairs, int base
                         const float* pred_dy, const float* pred_dx) {
   if (npred <= 0) return;
   const int nt = ((max_h + a.tile - 1) / a.tile) * ((max_w + a.tile - 1) / a.tile);
-  k_traj_verify<<<dim3((2 * nt + 63) / 64, npred), 64, 0, st>>>(
+  k_traj_verify<<<dim3((nt + kVerifyWarps - 1) / kVerifyWarps, npred), 32 * kVerifyWarps, 0, st>>>(
       d_fields, d_pairs, base, npred, d_grp, d_searched, d_tp, blur, a, dy_in, dx_in, pred_dy,
       pred_dx, mdy, mdx, sdy, sdx, best);
 }
@@ -1735,9 +1744,11 @@ void launch_me_confidence(const MeField* d_fields, const MePair* d_pairs, int np
                           float* dy, float* dx, float* conf, cudaStream_t st) {
   if (npairs <= 0) return;
   const int th = (max_h + a.tile - 1) / a.tile, tw = (max_w + a.tile - 1) / a.tile;
-  const int smem = 2 * th * tw * (int)sizeof(float);
-  k_me_confidence<<<npairs, 256, smem, st>>>(d_fields, d_pairs, npairs, blur, a, mdy, mdx, sdy, sdx,
-                                             best, dy, dx, conf);
+  const int nt = th * tw;
+  k_me_tile_stats<<<dim3((nt + kConfWarps - 1) / kConfWarps, npairs), 32 * kConfWarps, 0, st>>>(
+      d_fields, d_pairs, blur, a, best, dy, conf);
+  k_me_confidence<<<npairs, 256, nt * (int)sizeof(float), st>>>(d_pairs, a, nt, mdy, mdx, sdy, sdx,
+                                                                dy, dx, conf);
 }
 
 void launch_motion_cache(const int* d_gid, int npairs, int nt, int tiles_off, float* dy, float* dx,
@@ -1756,14 +1767,8 @@ void launch_coherence_gate(const MeField* d_fields, const MePair* d_pairs, int n
   const dim3 grid((max_w + 127) / 128, max_h, npairs);
   k_coh_terms<<<grid, 128, 0, st>>>(d_fields, d_pairs, npairs, a, b);
   // ComplexCoherence's four BoxBlur(r = 6) passes (temporal.cpp:186-189)
-  for (int c = 0; c < 4; ++c) {
-    float* ch = b.terms + c * b.chan_stride;
-    k_pair_blur_v<<<dim3((max_w + kBoxThreads - 1) / kBoxThreads, npairs), kBoxThreads, 0,
-                    st>>>(d_fields, d_pairs, npairs, ch,
-                                                                    b.tmp, b.pix_off, 6);
-    k_pair_blur_h<<<dim3((max_h + 31) / 32, npairs), 32, 0, st>>>(d_fields, d_pairs, npairs,
-                                                                 b.tmp, ch, b.pix_off, 6);
-  }
+  pair_blur(d_fields, d_pairs, npairs, max_h, max_w, b.terms, b.terms, b.pix_off, 4, b.chan_stride,
+            6, st);
   k_coh_apply<<<grid, 128, 0, st>>>(d_fields, d_pairs, npairs, b, gate);
 }
 

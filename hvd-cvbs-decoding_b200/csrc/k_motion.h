@@ -44,7 +44,6 @@ struct VecBuffers {
   float *c2, *c2_snap, *c2_snap2;    // fast-mode confidence tiles
   float* conf_tmp;                   // per-pixel scratch
   float* conf_px;                    // per-pixel confidence, per pair
-  size_t conf_bytes;
 };
 
 // Integer-SAD mode (me_mode 1): block x block tiles, exhaustive +-range.
@@ -55,7 +54,6 @@ struct SadArgs {
 
 struct SadBuffers {
   const float* luma;               // per field at MeField::y_off
-  int* vsum;                       // per field at MeField::t_off (vertical window sums)
   int* qblur;                      // per field at MeField::b_off (quantised, blurred luma)
   float *mdy, *mdx, *sdy, *sdx;    // per tile: integer vector, sub-pel offsets
   double *bestv, *s1, *s2, *npx;   // per tile: biased SSD (IRE^2), sums of A, pixel count
@@ -113,7 +111,6 @@ struct CohBuffers {
   const float* snap_dy;        // snapped tile vectors (pair i at i * tiles_off)
   const float* snap_dx;
   float* terms;                // 4 planes per pair: re, im, |chi_j|^2, |cw|^2
-  float* tmp;                  // one plane per pair
   float* conf_px;              // per-pixel confidence per pair (pix_off)
   const int64_t* pix_off;      // per-pair plane offset
   int64_t chan_stride;         // floats between the 4 channel blocks of terms

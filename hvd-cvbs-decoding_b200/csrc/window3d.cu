@@ -379,7 +379,6 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
   sad_a.tiles_off = nt;
   hvdg::SadBuffers sad_b;
   sad_b.luma = mb.luma;
-  sad_b.vsum = reinterpret_cast<int*>(mb.tmp);
   sad_b.qblur = reinterpret_cast<int*>(mb.blur);
   sad_b.mdy = mb.mdy;
   sad_b.mdx = mb.mdx;
@@ -550,7 +549,6 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
                                  mb.dy, mb.dx, mb.conf, s);
           S.launches += 1;
         }
-        vb.conf_bytes = sizeof(float) * plane * npairs;
         hvdg::launch_vectors(d_mf, d_mp, npairs, h, w, ma, vb, cfg.fast != 0, s);
         S.launches += 8;
         if (gate_cfg && !(cfg.fast && pass == 0)) {
@@ -560,7 +558,6 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
           cb.snap_dy = vb.snap_dy;
           cb.snap_dx = vb.snap_dx;
           cb.terms = at<float>(ctx, X(x_coh));
-          cb.tmp = vb.conf_tmp;
           cb.conf_px = vb.conf_px;
           cb.pix_off = d_pix_off;
           cb.chan_stride = coh_stride;
@@ -654,7 +651,6 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
         va.conf_px = at<float>(ctx, X(x_acpx));
         va.conf_tmp = at<float>(ctx, X(x_actmp));
         const int npairs_c = (int)mp.size();
-        va.conf_bytes = sizeof(float) * plane * npairs_c;
         if (npairs_c > 0) hvdg::launch_vectors(d_mf, d_mp, npairs_c, h, w, ma, va, false, s);
         hvdg::AnchorArgs aa;
         aa.fields = at<FieldDesc>(ctx, L.o_fields);
