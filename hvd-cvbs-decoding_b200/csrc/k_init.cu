@@ -23,6 +23,7 @@
 
 #include <cmath>
 
+#include "cluster_select.cuh"
 #include "hvdg_common.cuh"
 #include "k_init.h"
 #include "per_device.h"
@@ -904,20 +905,22 @@ __global__ void __launch_bounds__(256) k_init_blend(InitArgs a) {
 }
 
 // ---- auto chroma anisotropy (variational.cpp:130-196) ----------------------
-// Two CTAs (1024 threads) per field, one per axis: p98 of |delta| of 2-line
-// (NTSC) / 4-line (PAL) group averages, sampled at odd group rows and every
-// 3rd column, horizontal (axis 0) or vertical (axis 1) neighbour, exact k-th
-// element by radix select. The field's second CTA to finish maps the ratio
-// of the two to the split and writes mu_h, mu_v, mu_d.
-constexpr int kAnisoMax = 49152;
-__global__ void __launch_bounds__(1024) k_aniso(FieldDesc* fields, const float2* __restrict__ chi0) {
-  extern __shared__ float sm_an[];
-  __shared__ unsigned hist[256];
-  __shared__ unsigned bc[2];
+// A cluster of eight CTAs per field and axis: p98 of |delta| of 2-line (NTSC)
+// / 4-line (PAL) group averages, sampled at odd group rows and every 3rd
+// column, horizontal (axis 0) or vertical (axis 1) neighbour, exact k-th element
+// by radix selection among the samples in the cluster's registers. The field's
+// second cluster to finish maps the ratio of the two to the split and writes
+// mu_h, mu_v, mu_d. With one CTA per axis, its samples in shared memory, the
+// gather and the selection took 40 us on a lone NTSC field, this 15.
+constexpr int kAnisoPer = 6;
+constexpr int kAnisoMax = kSelCtas * kSelThreads * kAnisoPer;  // 49152
+__global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
+    k_aniso(FieldDesc* fields, const float2* __restrict__ chi0) {
+  __shared__ SelScratch sel;
   __shared__ int last;
-  FieldDesc& f = fields[blockIdx.x];
-  const int axis = blockIdx.y;
-  if (!(f.aniso_cfg > 0.0f)) {
+  FieldDesc& f = fields[blockIdx.x / kSelCtas];
+  const int axis = blockIdx.y, rank = blockIdx.x % kSelCtas;
+  if (!(f.aniso_cfg > 0.0f)) {  // the whole cluster
     const int group = f.is_pal ? 4 : 2;
     const int Hh = f.h / group;
     const int nt = Hh / 2;                // t = 1, 3, 5, ... < Hh
@@ -926,45 +929,38 @@ __global__ void __launch_bounds__(1024) k_aniso(FieldDesc* fields, const float2*
     if (n > kAnisoMax) n = kAnisoMax;     // geometry guard (the host rejects larger)
     const float2* c = chi0 + f.px_off;
     const float inv = 1.0f / (float)group;
-    // kAnisoBatch samples per thread and pass, all their loads issued before
-    // the first sum (one L2 round trip per batch, not per sample)
-    constexpr int kAnisoBatch = 4;
-    for (int i0 = threadIdx.x; i0 < n; i0 += kAnisoBatch * blockDim.x) {
-      float2 pv[kAnisoBatch][4], qv[kAnisoBatch][4];
+    const int share = (n + kSelCtas - 1) / kSelCtas, i0 = rank * share;
+    const int count = max(0, min(share, n - i0));
+    uint32_t key[kAnisoPer];
 #pragma unroll
-      for (int b = 0; b < kAnisoBatch; ++b) {
-        const int i = i0 + b * blockDim.x;
-        const int ti = i / nx, xi = i % nx;
-        const int tt = 1 + 2 * ti, x = 1 + 3 * xi;
+    for (int b = 0; b < kAnisoPer; ++b) {
+      key[b] = 0;
+      if ((int)threadIdx.x + b * kSelThreads < count) {
+        const int i = i0 + threadIdx.x + b * kSelThreads;
+        const int tt = 1 + 2 * (i / nx), x = 1 + 3 * (i % nx);
+        float2 pv[4], qv[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          pv[b][k] = qv[b][k] = make_float2(0.f, 0.f);
-          if (i < n && k < group) {
-            pv[b][k] = c[(int64_t)(group * tt + k) * f.pitch + x];
-            qv[b][k] = axis == 0 ? c[(int64_t)(group * tt + k) * f.pitch + x - 1]
-                                 : c[(int64_t)(group * (tt - 1) + k) * f.pitch + x];
-          }
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < kAnisoBatch; ++b) {
-        const int i = i0 + b * blockDim.x;
-        float2 p = make_float2(0.f, 0.f), q = p;
-        // the same order of additions as one sample at a time: k = 0, 1, ...
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < 4; ++k)
           if (k < group) {
-            p = cadd(p, pv[b][k]);
-            q = cadd(q, qv[b][k]);
+            pv[k] = c[(int64_t)(group * tt + k) * f.pitch + x];
+            qv[k] = axis == 0 ? c[(int64_t)(group * tt + k) * f.pitch + x - 1]
+                              : c[(int64_t)(group * (tt - 1) + k) * f.pitch + x];
           }
-        }
-        if (i < n) sm_an[i] = sqrtf(cnorm(csub(cscale(p, inv), cscale(q, inv))));
+        // the additions in the order k = 0, 1, ...
+        float2 p = make_float2(0.f, 0.f), q = p;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < group) {
+            p = cadd(p, pv[k]);
+            q = cadd(q, qv[k]);
+          }
+        key[b] = float_key(sqrtf(cnorm(csub(cscale(p, inv), cscale(q, inv)))));
       }
     }
-    __syncthreads();
-    const float p98 = n > 0 ? block_select_kth(sm_an, n, n - 1 - n / 50, hist, bc) : 0.f;
-    if (threadIdx.x == 0) f.aniso_p98[axis] = p98;
+    const float p98 = n > 0 ? cluster_select(key, count, n - 1 - n / 50, sel) : 0.f;
+    if (rank == 0 && threadIdx.x == 0) f.aniso_p98[axis] = p98;
   }
+  if (rank != 0) return;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -993,8 +989,6 @@ __global__ void __launch_bounds__(1024) k_aniso(FieldDesc* fields, const float2*
   f.mu_d = mu_d > 0.0f ? mu_d * scale : 0.0f;
 }
 
-constexpr int kAnisoSmem = kAnisoMax * (int)sizeof(float);
-
 static void configure_init_kernels_now() {
   float2 tw32[16];
   for (int k = 0; k < 16; ++k) {
@@ -1019,7 +1013,6 @@ static void configure_init_kernels_now() {
                        kLongColSmem);
   cudaFuncSetAttribute(k_sym_cols_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        kLongColSmem);
-  cudaFuncSetAttribute(k_aniso, cudaFuncAttributeMaxDynamicSharedMemorySize, kAnisoSmem);
 }
 
 // Kernel attributes and the twiddle constants, once per device.
@@ -1073,9 +1066,8 @@ void launch_init_filter_adjoint(const InitArgs& a, int total_prows, int total_cg
 }
 
 void launch_aniso(FieldDesc* d_fields, int n_fields, const float2* chi0, cudaStream_t st) {
-  const int smem = kAnisoSmem;
-  configure_init_kernels();
-  if (n_fields > 0) k_aniso<<<dim3(n_fields, 2), 1024, smem, st>>>(d_fields, chi0);
+  if (n_fields > 0)
+    k_aniso<<<dim3(n_fields * kSelCtas, 2), kSelThreads, 0, st>>>(d_fields, chi0);
 }
 
 int aniso_max_samples() { return kAnisoMax; }

@@ -1149,31 +1149,16 @@ __global__ void __launch_bounds__(kSadThreads, 6) k_sad_search(const MeField* __
   }
 }
 
-// Exact k-th smallest of v[0..n) (stable rank count), by the whole CTA.
-__device__ double block_kth_double(const double* v, int n, int k, double* slot) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double x = v[i];
-    int less = 0, eq_before = 0;
-    for (int j = 0; j < n; ++j) {
-      const double y = v[j];
-      less += y < x;
-      eq_before += (y == x) & (j < i);
-    }
-    if (less + eq_before == k) *slot = x;
-  }
-  __syncthreads();
-  const double r = *slot;
-  __syncthreads();
-  return r;
-}
-
 // MotionConfidence on the IRE scale from the exact integer statistics. One
 // CTA per pair.
-__global__ void __launch_bounds__(256) k_sad_confidence(const MeField* __restrict__ mf,
+// One block of 1024 threads per pair: the rank counts (nt^2 comparisons) bound it
+// (768 tiles, both middles: 64 us by 256 threads in two passes, 14 now).
+constexpr int kSadConfThreads = 1024;
+__global__ void __launch_bounds__(kSadConfThreads) k_sad_confidence(const MeField* __restrict__ mf,
                                                         const MePair* __restrict__ pairs,
                                                         SadArgs a, SadBuffers out) {
   extern __shared__ double sadc_sm[];
-  __shared__ double slot;
+  __shared__ double mid[2];
   const int p = blockIdx.x;
   const MeField mc = mf[pairs[p].cur];
   const int b = a.block;
@@ -1183,9 +1168,21 @@ __global__ void __launch_bounds__(256) k_sad_confidence(const MeField* __restric
   for (int t = threadIdx.x; t < nt; t += blockDim.x)
     ratios[t] = out.bestv[o + t] / fmax(1.0, out.npx[o + t]);
   __syncthreads();
+  // the two middle ratios by counting ranks, both in one pass
   const int k = nt / 2;
-  double med = block_kth_double(ratios, nt, k, &slot);
-  if (nt % 2 == 0) med = 0.5 * (med + block_kth_double(ratios, nt, k - 1, &slot));
+  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+    const double v = ratios[t];
+    int less = 0, eq = 0;
+#pragma unroll 8
+    for (int u = 0; u < nt; ++u) {
+      less += ratios[u] < v;
+      eq += ratios[u] == v;
+    }
+    if (less <= k && k < less + eq) mid[0] = v;
+    if (less <= k - 1 && k - 1 < less + eq) mid[1] = v;
+  }
+  __syncthreads();
+  const double med = nt % 2 == 0 ? 0.5 * (mid[0] + mid[1]) : mid[0];
   const double sc2 = (double)kQuantScale * (double)kQuantScale;
   for (int t = threadIdx.x; t < nt; t += blockDim.x) {
     const double npx = out.npx[o + t];
@@ -1215,7 +1212,7 @@ void launch_motion_sad(const MeField* d_fields, int nf, int max_h, int max_w,
     cudaFuncSetAttribute(k_sad_search, cudaFuncAttributeMaxDynamicSharedMemorySize, kSadMaxSmem);
   });
   k_sad_search<<<dim3(th * tw, npairs), kSadThreads, smem, st>>>(d_fields, d_pairs, b.qblur, a, b);
-  k_sad_confidence<<<npairs, 256, th * tw * (int)sizeof(double), st>>>(d_fields, d_pairs, a, b);
+  k_sad_confidence<<<npairs, kSadConfThreads, th * tw * (int)sizeof(double), st>>>(d_fields, d_pairs, a, b);
 }
 
 // ---------------------------------------------------------------------------

@@ -130,8 +130,13 @@ __device__ void tridiag_smooth(const double* d, const double* a, int n, double l
   __syncthreads();
 }
 
-// One CTA per field. blockDim = 256.
-__global__ void __launch_bounds__(256) k_burst_lockin(const PrepDesc* __restrict__ descs,
+// One CTA per field: a line per thread in the smoother and the angles, four
+// lines per warp in the burst sums (256 threads and a line per warp at a time:
+// 64 us for an NTSC field; 29 now, the FP64 divisions of the reduction's 18
+// steps and the angles' FP64 functions bounding it).
+constexpr int kLkThreads = 512;
+constexpr int kLkLines = 4;
+__global__ void __launch_bounds__(kLkThreads) k_burst_lockin(const PrepDesc* __restrict__ descs,
                                                       LockinOut out) {
   const PrepDesc p = descs[blockIdx.x];
   const int h = p.fh;
@@ -159,25 +164,46 @@ __global__ void __launch_bounds__(256) k_burst_lockin(const PrepDesc* __restrict
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int x0 = p.bx0, x1 = p.bx1, n = max(0, x1 - x0);
   // ---- per-line lock-in: z = mean((seg - mean) * exp(-i w0 x)) -------------
-  for (int y = warp; y < h; y += nwarps) {
-    double sum = 0.0;
-    for (int xx = x0 + lane; xx < x1; xx += 32) sum += (double)sample_ire(p, (int64_t)y * p.fw + xx);
-    sum = warp_allsum(sum);
-    const double mean = n > 0 ? sum / n : 0.0;
-    double ar = 0.0, ai = 0.0;
-    for (int xx = x0 + lane; xx < x1; xx += 32) {
-      const double v = (double)sample_ire(p, (int64_t)y * p.fw + xx) - mean;
-      const double2 ph = lo_phasor(p, xx);
-      ar += v * ph.x;
-      ai += v * ph.y;
+  // kLkLines lines of a warp at a time: their shuffle reductions and loads are
+  // independent chains
+  for (int yb = warp * kLkLines; yb < h; yb += nwarps * kLkLines) {
+    double mean[kLkLines], ar[kLkLines], ai[kLkLines];
+#pragma unroll
+    for (int q = 0; q < kLkLines; ++q) {
+      const int y = min(yb + q, h - 1);
+      mean[q] = 0.0;
+      for (int xx = x0 + lane; xx < x1; xx += 32)
+        mean[q] += (double)sample_ire(p, (int64_t)y * p.fw + xx);
     }
-    ar = warp_allsum(ar);
-    ai = warp_allsum(ai);
-    if (lane == 0) {
-      zr[y] = n > 0 ? ar / n : 0.0;
-      zi[y] = n > 0 ? ai / n : 0.0;
-      amp[y] = sqrt(zr[y] * zr[y] + zi[y] * zi[y]);
+#pragma unroll
+    for (int q = 0; q < kLkLines; ++q) {
+      mean[q] = warp_allsum(mean[q]);
+      mean[q] = n > 0 ? mean[q] / n : 0.0;
     }
+#pragma unroll
+    for (int q = 0; q < kLkLines; ++q) {
+      const int y = min(yb + q, h - 1);
+      ar[q] = ai[q] = 0.0;
+      for (int xx = x0 + lane; xx < x1; xx += 32) {
+        const double v = (double)sample_ire(p, (int64_t)y * p.fw + xx) - mean[q];
+        const double2 ph = lo_phasor(p, xx);
+        ar[q] += v * ph.x;
+        ai[q] += v * ph.y;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kLkLines; ++q) {
+      ar[q] = warp_allsum(ar[q]);
+      ai[q] = warp_allsum(ai[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kLkLines; ++q)
+      if (lane == q && yb + q < h) {
+        const int y = yb + q;
+        zr[y] = n > 0 ? ar[q] / n : 0.0;
+        zi[y] = n > 0 ? ai[q] / n : 0.0;
+        amp[y] = sqrt(zr[y] * zr[y] + zi[y] * zi[y]);
+      }
   }
   __syncthreads();
   // good lines: amplitude above 20 % of the field's maximum
@@ -419,7 +445,7 @@ void configure_prep_kernels() {
 
 void launch_burst_lockin(const PrepDesc* d_descs, int n, LockinOut out, cudaStream_t st) {
   configure_prep_kernels();
-  if (n > 0) k_burst_lockin<<<n, 256, kLockinSmem, st>>>(d_descs, out);
+  if (n > 0) k_burst_lockin<<<n, kLkThreads, kLockinSmem, st>>>(d_descs, out);
 }
 void launch_burst_amplitude(const PrepDesc* d_descs, int n, float* d_amp, cudaStream_t st) {
   if (n > 0) k_burst_amplitude<<<n, kAmpThreads, 0, st>>>(d_descs, d_amp);

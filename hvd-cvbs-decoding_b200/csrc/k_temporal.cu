@@ -15,6 +15,7 @@
 // arithmetic follows the reference's order.
 #include <cuda_runtime.h>
 
+#include "cluster_select.cuh"
 #include "hvdg_common.cuh"
 #include "k_temporal.h"
 #include "per_device.h"
@@ -50,6 +51,43 @@ __global__ void __launch_bounds__(1024) k_noise(const FieldDesc* __restrict__ fi
   __syncthreads();
   const float q = block_select_kth(d, n, n / 4, hist, bc);
   if (threadIdx.x == 0) sigma[blockIdx.x] = q / 0.3186f / sqrtf(6.0f);
+}
+
+// The same with a field's samples in the registers of a cluster (fields of up
+// to kNoiseMax samples; wider planes keep the kernel above): 437 -> 28 us for
+// the two selections of an NTSC field.
+constexpr int kNoisePer = 36;
+constexpr int kNoiseMax = kSelCtas * kSelThreads * kNoisePer;
+__global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
+    k_noise_cluster(const FieldDesc* __restrict__ fields, const float* __restrict__ S,
+                    float* __restrict__ sigma) {
+  __shared__ SelScratch sel;
+  const int field = blockIdx.x / kSelCtas, r = blockIdx.x % kSelCtas;
+  const FieldDesc& f = fields[field];
+  const int w = f.w, h = f.h, pitch = f.pitch;
+  if (w <= 8 || h <= 0) {  // the whole cluster
+    if (r == 0 && threadIdx.x == 0) sigma[field] = 0.0f;
+    return;
+  }
+  const int nx = w - 8, n = h * nx;
+  const int share = (n + kSelCtas - 1) / kSelCtas, i0 = r * share;
+  const int count = max(0, min(share, n - i0));
+  const float* s = S + f.px_off;
+  uint32_t key[kNoisePer];
+#pragma unroll
+  for (int q = 0; q < kNoisePer; ++q) {
+    const int i = i0 + threadIdx.x + q * kSelThreads;
+    key[q] = 0;
+    if ((int)threadIdx.x + q * kSelThreads < count) {
+      const float* row = s + (int64_t)(i / nx) * pitch + i % nx;
+      key[q] = float_key(row[0] - 2.0f * row[4] + row[8]);
+    }
+  }
+  const float med = cluster_select(key, count, n / 2, sel);
+#pragma unroll
+  for (int q = 0; q < kNoisePer; ++q) key[q] = float_key(fabsf(key_float(key[q]) - med));
+  const float q4 = cluster_select(key, count, n / 4, sel);
+  if (r == 0 && threadIdx.x == 0) sigma[field] = q4 / 0.3186f / sqrtf(6.0f);
 }
 
 // ---- envelope gate --------------------------------------------------------------
@@ -197,6 +235,71 @@ __global__ void __launch_bounds__(1024) k_env_floor(const FieldDesc* __restrict_
     }
   }
   if (threadIdx.x == 0) floor2[blockIdx.x] = 2.25f * med * med;
+}
+
+// The same from the registers of a cluster, for up to kFloorMax samples.
+constexpr int kFloorPer = 5;
+constexpr int kFloorMax = kSelCtas * kSelThreads * kFloorPer;
+__global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
+    k_env_floor_cluster(const FieldDesc* __restrict__ fields, const int* __restrict__ list,
+                        const float* __restrict__ vraw, float* __restrict__ floor2) {
+  namespace cg = cooperative_groups;
+  __shared__ SelScratch sel;
+  __shared__ unsigned below[kSelCtas], top[kSelCtas], wb[32], wt[32];
+  cg::cluster_group cl = cg::this_cluster();
+  const int fi = list[blockIdx.x / kSelCtas], r = blockIdx.x % kSelCtas;
+  const FieldDesc& f = fields[fi];
+  const int w = f.w, n = (int)(((int64_t)f.h * w + 6) / 7);
+  const int share = (n + kSelCtas - 1) / kSelCtas, i0 = r * share;
+  const int count = max(0, min(share, n - i0));
+  uint32_t key[kFloorPer];
+#pragma unroll
+  for (int q = 0; q < kFloorPer; ++q) {
+    key[q] = 0;
+    if ((int)threadIdx.x + q * kSelThreads < count) {
+      const int flat = (i0 + threadIdx.x + q * kSelThreads) * 7;
+      key[q] = float_key(vraw[f.px_off + (int64_t)(flat / w) * f.pitch + flat % w]);
+    }
+  }
+  float med = 0.0f;
+  if (n > 0) {
+    med = cluster_select(key, count, n / 2, sel);
+    if (n % 2 == 0) {
+      // the value of rank n/2 - 1: the largest one below med when exactly n/2
+      // lie below it, else med itself
+      const uint32_t mk = float_key(med);
+      unsigned cnt = 0, mx = 0;
+#pragma unroll
+      for (int q = 0; q < kFloorPer; ++q)
+        if ((int)threadIdx.x + q * kSelThreads < count && key[q] < mk) {
+          ++cnt;
+          mx = max(mx, key[q]);
+        }
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      if ((threadIdx.x & 31) == 0) {
+        wb[threadIdx.x >> 5] = cnt;
+        wt[threadIdx.x >> 5] = mx;
+      }
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        cnt = __reduce_add_sync(0xffffffffu, wb[threadIdx.x]);
+        mx = __reduce_max_sync(0xffffffffu, wt[threadIdx.x]);
+        if (threadIdx.x < kSelCtas) {
+          *cl.map_shared_rank(&below[r], threadIdx.x) = cnt;
+          *cl.map_shared_rank(&top[r], threadIdx.x) = mx;
+        }
+      }
+      cl.sync();
+      unsigned b = 0, t = 0;
+      for (int q = 0; q < kSelCtas; ++q) {
+        b += below[q];
+        t = max(t, top[q]);
+      }
+      med = 0.5f * (med + (b == (unsigned)(n / 2) ? key_float(t) : med));
+    }
+  }
+  if (r == 0 && threadIdx.x == 0) floor2[blockIdx.x / kSelCtas] = 2.25f * med * med;
 }
 
 // (4) floored envelope, extremum factor, final odd-offset gate
@@ -374,9 +477,13 @@ void launch_amb_pairs(const FieldDesc* d_fields, int npairs, int stride, int nyi
   k_amb_pairs<<<npairs, 32, 0, st>>>(nyi, nx, E, amb, ok);
 }
 
-void launch_noise(const FieldDesc* d_fields, int nf, const float* S, float* scratch,
+void launch_noise(const FieldDesc* d_fields, int nf, int h, int w, const float* S, float* scratch,
                   const int64_t* scratch_off, float* sigma, cudaStream_t st) {
-  if (nf > 0) k_noise<<<nf, 1024, 0, st>>>(d_fields, S, scratch, scratch_off, sigma);
+  if (nf <= 0) return;
+  if ((int64_t)h * w <= kNoiseMax)
+    k_noise_cluster<<<nf * kSelCtas, kSelThreads, 0, st>>>(d_fields, S, sigma);
+  else
+    k_noise<<<nf, 1024, 0, st>>>(d_fields, S, scratch, scratch_off, sigma);
 }
 
 void launch_envelope(const FieldDesc* d_fields, const int* d_list, int n, int max_h, int max_w,
@@ -393,7 +500,10 @@ void launch_envelope(const FieldDesc* d_fields, const int* d_list, int n, int ma
   k_env_smooth<<<dim3((max_h + kSmoothRows - 1) / kSmoothRows, n, 2), 256,
                  sizeof(float) * kSmoothRows * smooth_stride(max_w), st>>>(
       d_fields, d_list, e.gmag, e.lapmag, e.vraw, e.traw);
-  k_env_floor<<<n, 1024, 0, st>>>(d_fields, d_list, e.vraw, e.scratch, e.scratch_off, e.floor2);
+  if (((int64_t)max_h * max_w + 6) / 7 <= kFloorMax)
+    k_env_floor_cluster<<<n * kSelCtas, kSelThreads, 0, st>>>(d_fields, d_list, e.vraw, e.floor2);
+  else
+    k_env_floor<<<n, 1024, 0, st>>>(d_fields, d_list, e.vraw, e.scratch, e.scratch_off, e.floor2);
   k_env_gate<<<dim3((max_w + 127) / 128, max_h, n), 128, 0, st>>>(
       d_fields, d_list, e.vraw, e.traw, e.floor2, e2, floor_max, e.gate);
 }

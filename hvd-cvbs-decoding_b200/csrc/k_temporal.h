@@ -31,7 +31,8 @@ struct EnvBuffers {
 void launch_amb_pairs(const FieldDesc* d_fields, int npairs, int stride, int nyi, int nx,
                       const float* S, const float4* lineph, const float2* colph, float nr_eps,
                       double* E, float* amb, int* ok, cudaStream_t st);
-void launch_noise(const FieldDesc* d_fields, int nf, const float* S, float* scratch,
+// h, w: the fields' largest active size
+void launch_noise(const FieldDesc* d_fields, int nf, int h, int w, const float* S, float* scratch,
                   const int64_t* scratch_off, float* sigma, cudaStream_t st);
 void launch_envelope(const FieldDesc* d_fields, const int* d_list, int n, int max_h, int max_w,
                      const float* Y, const float2* X, const EnvBuffers& e, float e2,

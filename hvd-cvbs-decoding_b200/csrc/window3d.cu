@@ -228,7 +228,7 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "H2D window tables");
 
   // ---- noise self-calibration (sequence.cpp:437-449) ----
-  hvdg::launch_noise(at<FieldDesc>(ctx, L.o_fields), nf, at<float>(ctx, L.o_S),
+  hvdg::launch_noise(at<FieldDesc>(ctx, L.o_fields), nf, h, w, at<float>(ctx, L.o_S),
                      at<float>(ctx, X(x_nscr)), d_nscr_off, d_sigma, s);
   std::vector<float> sig(nf);
   e = cudaMemcpyAsync(sig.data(), d_sigma, sizeof(float) * nf, cudaMemcpyDeviceToHost, s);
