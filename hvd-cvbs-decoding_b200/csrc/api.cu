@@ -982,13 +982,8 @@ hvdg_status hvdg_decode_fields_adjoint(hvdg_ctx* ctx, const hvdg_field_in* field
   cudaSetDevice(ctx->device);
   const int iters = adjoint_cg_iterations > 0 ? adjoint_cg_iterations : 300;
   for (int i = 0; i < 4; ++i) scalar_bar[i] = 0.0;
-  for (int i = 0; i < n; ++i) {
-    const hvdg_status st = decode_adjoint_field(ctx, fields[i], *cfg, y_bar[i], chi_bar[i],
-                                                samples_bar[i], scalar_bar, iters,
-                                                out ? &out[i] : nullptr, diag);
-    if (st != HVDG_OK) return st;
-  }
-  return HVDG_OK;
+  return decode_adjoint_fields(ctx, fields, n, *cfg, y_bar, chi_bar, samples_bar, scalar_bar, iters,
+                               out, diag);
 }
 
 }  // extern "C"

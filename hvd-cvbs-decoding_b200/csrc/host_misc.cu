@@ -150,38 +150,64 @@ hvdg_status estimate_motion_sad(hvdg_ctx* ctx, const float* y_ref, const float* 
   return HVDG_OK;
 }
 
-// Decode adjoint of one 2-D field (no reference counterpart): forward with
-// the IRLS iterates checkpointed (one solver launch per outer, so chi_o and
-// the weights W(chi_o) can be kept), then the reverse sweep over the outers
-// (an adjoint CG solve per outer in the same persistent solver, weights
-// frozen, right-hand side injected as a constant gradient term), then the
-// HolographicInit adjoint and the crop / level transposes.
-hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const hvdg_config& cfg,
-                                 const float* y_bar, const float* chi_bar, float* samples_bar,
+namespace {
+
+// Fields of one adjoint launch: bounded in number and in the device memory
+// that their checkpoints take (8 + 16 bytes per pixel and outer, beside about
+// 230 of working planes).
+constexpr int kAdjMaxFields = 32;
+constexpr double kAdjMaxBytes = 4e9, kAdjBytesPerPx = 230.0, kAdjBytesPerOuter = 24.0;
+
+struct AdjBudget {
+  int n_outer, n_inner;
+};
+AdjBudget adjoint_budget(const hvdg_field_in& f, const hvdg_config& cfg) {
+  AdjBudget b;
+  b.n_outer = std::max(1, f.irls_outer > 0 ? f.irls_outer : cfg.irls_outer);
+  const int cg_cfg = f.cg_iterations >= 0 ? f.cg_iterations : cfg.cg_iterations;
+  const int cg_total = cfg.fast ? cg_cfg * 2 / 3 : cg_cfg;
+  b.n_inner = std::max(1, cg_total / b.n_outer);
+  return b;
+}
+
+// Decode adjoint of n 2-D fields of one geometry and one budget (no reference
+// counterpart): forward with the IRLS iterates checkpointed (one solver launch
+// per outer, so chi_o and the weights W(chi_o) can be kept), then the reverse
+// sweep over the outers (an adjoint CG solve per outer in the same solver,
+// weights frozen, right-hand side injected as a constant gradient term), then
+// the HolographicInit adjoint and the crop / level transposes. The fields go
+// through each launch together: alone on the chip a field's CG sweep is bound
+// by the exchange between its CTAs, and several fields share that time.
+hvdg_status decode_adjoint_chunk(hvdg_ctx* ctx, const hvdg_field_in* fields, int n,
+                                 const hvdg_config& cfg, const float* const* y_bar,
+                                 const float* const* chi_bar, float* const* samples_bar,
                                  double* scalar_bar, int adj_iters, hvdg_field_out* out,
                                  hvdg_diag* diag) {
-  const hvdg_geometry& g = *fi.geometry;
+  const hvdg_geometry& g = *fields[0].geometry;
   const int h = last_active_line(g) - g.first_active_field_line;
   const int w = g.active_video_end - g.active_video_start;
   const int pitch = (w + hvdg::kStrip - 1) / hvdg::kStrip * hvdg::kStrip;
   const int pad = std::min(hvdg::kInitPad, h - 1 > 0 ? h - 1 : 0);
   const int hp = h + 2 * pad;
-  const int64_t plane = (int64_t)h * pitch;
-  const int64_t rplane = (int64_t)hp * pitch;
+  const int64_t field_px = (int64_t)h * pitch;
+  const int64_t plane = field_px * n;
+  const int64_t rplane = (int64_t)hp * pitch * n;
+  const size_t n_samples = (size_t)g.field_height * g.field_width;
   // the forward's budget, one outer per solver launch
-  const int n_outer = std::max(1, fi.irls_outer > 0 ? fi.irls_outer : cfg.irls_outer);
-  const int cg_cfg = fi.cg_iterations >= 0 ? fi.cg_iterations : cfg.cg_iterations;
-  const int cg_total = cfg.fast ? cg_cfg * 2 / 3 : cg_cfg;
-  const int n_inner = std::max(1, cg_total / n_outer);
+  const AdjBudget bud = adjoint_budget(fields[0], cfg);
+  const int n_outer = bud.n_outer, n_inner = bud.n_inner;
   hvdg_config c1 = cfg;
   c1.irls_outer = 1;
   c1.cg_iterations = n_inner;
   c1.fast = 0;
   c1.cg_tol = cfg.cg_tol > 0.0f ? cfg.cg_tol : (cfg.fast ? 0.10f : 0.02f);
-  hvdg_field_in f1 = fi;
-  f1.irls_outer = 1;
-  f1.cg_iterations = n_inner;
+  std::vector<hvdg_field_in> f1(fields, fields + n);
+  for (hvdg_field_in& f : f1) {
+    f.irls_outer = 1;
+    f.cg_iterations = n_inner;
+  }
   hvdg::AdjGeom ag;
+  ag.n = n;
   ag.h = h;
   ag.w = w;
   ag.pitch = pitch;
@@ -206,12 +232,13 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
   const size_t x_ai = take(sizeof(float2) * plane * 5);
   const size_t x_ain = take(sizeof(float2) * rplane * 2);
   const size_t x_aout = take(sizeof(float2) * rplane * 2);
-  const size_t x_part = take(sizeof(double) * 4 * nb);
-  const size_t x_acc = take(sizeof(double) * 4);
-  const size_t x_smp = take(sizeof(float) * (size_t)g.field_height * g.field_width);
+  const size_t x_part = take(sizeof(double) * 4 * nb * n);
+  const size_t x_acc = take(sizeof(double) * 4 * n);
+  const size_t x_af = take(sizeof(hvdg::AdjField) * n);
+  const size_t x_smp = take(sizeof(float) * n_samples * n);
   RunOpts opt;
   Staged S;
-  hvdg_status st = stage_upload(ctx, &f1, 1, &c1, opt, xo, S);
+  hvdg_status st = stage_upload(ctx, f1.data(), n, &c1, opt, xo, S);
   if (st != HVDG_OK) return st;
   const Layout& L = S.b.L;
   auto X = [&](size_t off) { return S.extra + off; };
@@ -232,11 +259,12 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(ck, at<float2>(ctx, L.o_X0), sizeof(float2) * plane, cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint checkpoints");
-  hvdg::launch_aniso(at<FieldDesc>(ctx, L.o_fields), 1, at<float2>(ctx, L.o_X0), s);
+  hvdg::launch_aniso(at<FieldDesc>(ctx, L.o_fields), n, at<float2>(ctx, L.o_X0), s);
   // ---- forward, one outer per launch ----
   hvdg::SolverArgs sa = solver_args(ctx, S);
   sa.keep_w = 1;  // each outer's weights are checkpointed
   int cg_run = 0;
+  std::vector<FieldCtl> ctl(n);
   for (int o = 0; o < n_outer; ++o) {
     stage_reset(ctx, S);
     e = launch_solve(ctx, S, sa, S.b.rg, false);
@@ -247,9 +275,9 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
       e = cudaMemcpyAsync(wk + o * plane, at<float4>(ctx, L.o_W), sizeof(float4) * plane,
                           cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint checkpoints");
-    FieldCtl ctl;
     int flags[4];
-    e = cudaMemcpyAsync(&ctl, at<FieldCtl>(ctx, L.o_ctl), sizeof(ctl), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(ctl.data(), at<FieldCtl>(ctx, L.o_ctl), sizeof(FieldCtl) * n,
+                        cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(flags, at<int>(ctx, L.o_flags), sizeof(flags), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -262,36 +290,48 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
       ctx->last_error = "device-side bounded wait expired in the solver";
       return HVDG_ERR_DEVICE_TIMEOUT;
     }
-    cg_run += ctl.cg_iters;
+    for (const FieldCtl& c : ctl) cg_run += c.cg_iters;
   }
-  if (out && (out->luma || out->chroma)) {
-    if (out->luma)
-      e = cudaMemcpy2DAsync(out->luma, sizeof(float) * w, at<float>(ctx, L.o_Y), sizeof(float) * pitch,
-                            sizeof(float) * w, h, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && out->chroma)
-      e = cudaMemcpy2DAsync(out->chroma, sizeof(float2) * w, at<float2>(ctx, L.o_X0),
-                            sizeof(float2) * pitch, sizeof(float2) * w, h, cudaMemcpyDeviceToHost, s);
+  for (int i = 0; out && i < n; ++i) {
+    e = cudaSuccess;
+    if (out[i].luma)
+      e = cudaMemcpy2DAsync(out[i].luma, sizeof(float) * w, at<float>(ctx, L.o_Y) + field_px * i,
+                            sizeof(float) * pitch, sizeof(float) * w, h, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && out[i].chroma)
+      e = cudaMemcpy2DAsync(out[i].chroma, sizeof(float2) * w,
+                            at<float2>(ctx, L.o_X0) + field_px * i, sizeof(float2) * pitch,
+                            sizeof(float2) * w, h, cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint forward outputs");
   }
   // ---- reverse sweep ----
-  FieldDesc fd;
-  e = cudaMemcpyAsync(&fd, at<FieldDesc>(ctx, L.o_fields), sizeof(fd), cudaMemcpyDeviceToHost, s);
+  std::vector<FieldDesc> fd(n);
+  e = cudaMemcpyAsync(fd.data(), at<FieldDesc>(ctx, L.o_fields), sizeof(FieldDesc) * n,
+                      cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint field descriptor");
-  hvdg::AdjScalars sc;
-  sc.eps = cfg.charbonnier_eps;
-  sc.eps_c = cfg.chroma_eps;
-  sc.k = cfg.structure_coupling;
-  sc.mu_h = fd.mu_h;
-  sc.mu_v = fd.mu_v;
-  sc.aniso = cfg.lambda_c != 0.0f ? fd.mu_h / cfg.lambda_c : 1.0f;
-  FieldDesc fa = fd;
-  fa.n_outer = 1;
-  fa.n_inner = adj_iters;
-  fa.n_phases = 2 + adj_iters + 1;
-  fa.cg_tol = 1e-6f;
-  fa.adj_flags = hvdg::kAdjFixedW | hvdg::kAdjExtB;
-  fa.has_nbr = 0;
+  std::vector<hvdg::AdjField> af(n);
+  for (int i = 0; i < n; ++i) {
+    hvdg::AdjScalars& sc = af[i].sc;
+    sc.eps = cfg.charbonnier_eps;
+    sc.eps_c = cfg.chroma_eps;
+    sc.k = cfg.structure_coupling;
+    sc.mu_h = fd[i].mu_h;
+    sc.mu_v = fd[i].mu_v;
+    sc.aniso = cfg.lambda_c != 0.0f ? fd[i].mu_h / cfg.lambda_c : 1.0f;
+    const float cpi = fields[i].sample_type == HVDG_SAMPLES_F32_IRE
+                          ? 1.0f
+                          : (fields[i].white_level - fields[i].blanking_level) / 100.0f;
+    af[i].inv_cpi = 1.0f / cpi;
+    af[i].sigma = 1.0f;
+    af[i].active = 1;
+    FieldDesc& fa = fd[i];
+    fa.n_outer = 1;
+    fa.n_inner = adj_iters;
+    fa.n_phases = 2 + adj_iters + 1;
+    fa.cg_tol = 1e-6f;
+    fa.adj_flags = hvdg::kAdjFixedW | hvdg::kAdjExtB;
+    fa.has_nbr = 0;
+  }
   float* zero = at<float>(ctx, X(x_zero));
   float2* B = at<float2>(ctx, X(x_B));
   float* yb = at<float>(ctx, X(x_yb));
@@ -300,42 +340,53 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
   float2* pa = at<float2>(ctx, X(x_pa));
   double* part = at<double>(ctx, X(x_part));
   double* acc = at<double>(ctx, X(x_acc));
+  hvdg::AdjField* d_af = at<hvdg::AdjField>(ctx, X(x_af));
   e = cudaMemsetAsync(zero, 0, sizeof(float) * plane, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(yb, 0, sizeof(float) * plane, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(cb, 0, sizeof(float2) * plane, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(double) * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(double) * 4 * n, s);
+  for (int i = 0; i < n && e == cudaSuccess; ++i) {
+    e = cudaMemcpy2DAsync(yb + field_px * i, sizeof(float) * pitch, y_bar[i], sizeof(float) * w,
+                          sizeof(float) * w, h, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpy2DAsync(cb + field_px * i, sizeof(float2) * pitch, chi_bar[i],
+                            sizeof(float2) * w, sizeof(float2) * w, h, cudaMemcpyHostToDevice, s);
+  }
   if (e == cudaSuccess)
-    e = cudaMemcpy2DAsync(yb, sizeof(float) * pitch, y_bar, sizeof(float) * w, sizeof(float) * w, h,
-                          cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpy2DAsync(cb, sizeof(float2) * pitch, chi_bar, sizeof(float2) * w,
-                          sizeof(float2) * w, h, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(at<FieldDesc>(ctx, L.o_fields), &fa, sizeof(fa), cudaMemcpyHostToDevice, s);
+    e = cudaMemcpyAsync(at<FieldDesc>(ctx, L.o_fields), fd.data(), sizeof(FieldDesc) * n,
+                        cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint cotangents");
   hvdg::launch_adj_output(ag, yb, sb, cb, s);
   hvdg::SolverArgs sadj = sa;
   sadj.keep_w = 0;
   sadj.S = zero;
   sadj.B = B;
-  sadj.n_phases = fa.n_phases;
-  std::vector<double> np(nb);
+  sadj.n_phases = fd[0].n_phases;
+  std::vector<double> np((size_t)nb * n);
   int adj_run = 0;
   for (int o = n_outer - 1; o >= 0; --o) {
-    // scale the right-hand side to unit rms (the solver's absolute exit is
+    // scale each right-hand side to unit rms (the solver's absolute exit is
     // relative to the field size)
     hvdg::launch_adj_norm(ag, cb, part, s);
-    e = cudaMemcpyAsync(np.data(), part, sizeof(double) * nb, cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(np.data(), part, sizeof(double) * nb * n, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint norm");
-    double ss = 0.0;
-    for (int i = 0; i < nb; ++i) ss += np[i];
-    if (!(ss > 0.0)) {
+    int n_active = 0;
+    for (int i = 0; i < n; ++i) {
+      if (!af[i].active) continue;
+      double ss = 0.0;
+      for (int j = 0; j < nb; ++j) ss += np[(size_t)nb * i + j];
       // zero cotangent: every contribution of this and earlier outers is zero
-      break;
+      af[i].active = ss > 0.0;
+      if (!af[i].active) continue;
+      af[i].sigma = (float)(1.0 / std::sqrt(ss / ((double)h * w)));
+      ++n_active;
     }
-    const float sigma = (float)(1.0 / std::sqrt(ss / ((double)h * w)));
-    hvdg::launch_adj_rhs(ag, cb, sigma, B, s);
+    // (also before the break: the samples' levels are read from the table)
+    e = cudaMemcpyAsync(d_af, af.data(), sizeof(hvdg::AdjField) * n, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint solve setup");
+    if (n_active == 0) break;
+    hvdg::launch_adj_rhs(ag, d_af, cb, B, s);
     e = cudaMemcpyAsync(at<float4>(ctx, L.o_W), wk + o * plane, sizeof(float4) * plane,
                         cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(at<float2>(ctx, L.o_X0), 0, sizeof(float2) * plane, s);
@@ -346,7 +397,6 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
     hvdg::AdjOuter ao;
     ao.S = at<float>(ctx, L.o_S);
     ao.lam = at<float2>(ctx, L.o_X0);
-    ao.inv_sigma = 1.0f / sigma;
     ao.chi1 = ck + (o + 1) * plane;
     ao.chi0 = ck + o * plane;
     ao.W = wk + o * plane;
@@ -355,10 +405,10 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
     ao.A1 = pa + 2 * plane;
     ao.A2 = pa + 3 * plane;
     ao.partials = part;
-    hvdg::launch_adj_outer(ag, sc, ao, acc, sb, cb, s);
-    FieldCtl ctl;
+    hvdg::launch_adj_outer(ag, d_af, ao, acc, sb, cb, s);
     int flags[4];
-    e = cudaMemcpyAsync(&ctl, at<FieldCtl>(ctx, L.o_ctl), sizeof(ctl), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(ctl.data(), at<FieldCtl>(ctx, L.o_ctl), sizeof(FieldCtl) * n,
+                        cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(flags, at<int>(ctx, L.o_flags), sizeof(flags), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -367,7 +417,8 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
       ctx->last_error = "device-side bounded wait expired in the adjoint solver";
       return HVDG_ERR_DEVICE_TIMEOUT;
     }
-    adj_run += ctl.cg_iters;
+    for (int i = 0; i < n; ++i)
+      if (af[i].active) adj_run += ctl[i].cg_iters;
   }
   // ---- HolographicInit adjoint (chibar now holds the cotangent of chi_0) ----
   float2* ai = at<float2>(ctx, X(x_ai));
@@ -392,24 +443,61 @@ hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const h
   fa_init.adj_out = aout;
   hvdg::launch_init_filter_adjoint(fa_init, L.total_prows, L.total_cgroups, s);
   hvdg::launch_adj_fold(ag, aout, sb, s);
-  const float cpi = fi.sample_type == HVDG_SAMPLES_F32_IRE
-                        ? 1.0f
-                        : (fi.white_level - fi.blanking_level) / 100.0f;
   float* smp = at<float>(ctx, X(x_smp));
-  hvdg::launch_adj_samples(ag, sb, 1.0f / cpi, g.field_height, g.field_width,
-                           g.first_active_field_line, g.active_video_start, smp, s);
-  double accv[4];
+  hvdg::launch_adj_samples(ag, d_af, sb, g.field_height, g.field_width, g.first_active_field_line,
+                           g.active_video_start, smp, s);
+  std::vector<double> accv(4 * (size_t)n);
   e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(samples_bar, smp, sizeof(float) * (size_t)g.field_height * g.field_width,
+  for (int i = 0; i < n && e == cudaSuccess; ++i)
+    e = cudaMemcpyAsync(samples_bar[i], smp + n_samples * i, sizeof(float) * n_samples,
                         cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(accv, acc, sizeof(accv), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(accv.data(), acc, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "adjoint outputs");
-  for (int i = 0; i < 4; ++i) scalar_bar[i] += accv[i];
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < 4; ++i) scalar_bar[i] += accv[4 * j + i];
   if (diag) {
     diag->cg_iterations_run += cg_run + adj_run;
-    diag->kernel_launches += 8 + n_outer * 6 + 12;
+    diag->kernel_launches += 8 + n_outer * 7 + 12;
+  }
+  return HVDG_OK;
+}
+
+}  // namespace
+
+// Consecutive fields of one geometry and one budget go through together, as
+// many as their checkpoints leave room for.
+hvdg_status decode_adjoint_fields(hvdg_ctx* ctx, const hvdg_field_in* fields, int n,
+                                  const hvdg_config& cfg, const float* const* y_bar,
+                                  const float* const* chi_bar, float* const* samples_bar,
+                                  double* scalar_bar, int adj_iters, hvdg_field_out* out,
+                                  hvdg_diag* diag) {
+  for (int i = 0; i < n;) {
+    const hvdg_geometry& g = *fields[i].geometry;
+    const AdjBudget b = adjoint_budget(fields[i], cfg);
+    const double px = (double)(last_active_line(g) - g.first_active_field_line) *
+                      (g.active_video_end - g.active_video_start);
+    const int cap = (int)std::min(
+        (double)kAdjMaxFields,
+        std::max(1.0, kAdjMaxBytes / (px * (kAdjBytesPerPx + kAdjBytesPerOuter * b.n_outer))));
+    int m = 1;
+    while (i + m < n && m < cap) {
+      const AdjBudget bm = adjoint_budget(fields[i + m], cfg);
+      const hvdg_geometry& gm = *fields[i + m].geometry;
+      if (bm.n_outer != b.n_outer || bm.n_inner != b.n_inner || geom_key(gm) != geom_key(g) ||
+          gm.field_height != g.field_height)
+        break;
+      ++m;
+    }
+    auto run = [&](int k) {
+      return decode_adjoint_chunk(ctx, fields + i, k, cfg, y_bar + i, chi_bar + i, samples_bar + i,
+                                  scalar_bar, adj_iters, out ? out + i : nullptr, diag);
+    };
+    hvdg_status st = run(m);
+    if (st == HVDG_ERR_OUT_OF_MEMORY && m > 1) st = run(m = 1);
+    if (st != HVDG_OK) return st;
+    i += m;
   }
   return HVDG_OK;
 }

@@ -29,8 +29,13 @@ namespace {
 
 constexpr int kBX = 32, kBY = 8;
 
+// index of this block's field's plane
+__device__ __forceinline__ int64_t plane_of(const AdjGeom& g) {
+  return (int64_t)blockIdx.z * g.h * g.pitch;
+}
+
 __device__ __forceinline__ float2 car(const AdjGeom& g, int y, int x) {
-  const float4 L = __ldg(g.line_phasor + y);
+  const float4 L = __ldg(g.line_phasor + (int64_t)blockIdx.z * g.h + y);
   return carrier(make_float2(L.x, L.y), __ldg(g.col_phasor + x), L.z);
 }
 
@@ -75,7 +80,7 @@ __global__ void k_adj_output(AdjGeom g, const float* __restrict__ ybar, float* _
                              float2* __restrict__ chib) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= g.w || y >= g.h) return;
-  const int64_t o = (int64_t)y * g.pitch + x;
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
   const float yb = ybar[o];
   const float2 c = car(g, y, x);
   sbar[o] = yb;
@@ -90,37 +95,43 @@ __global__ void k_adj_norm(AdjGeom g, const float2* __restrict__ chib, double* _
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   double v[1] = {0.0};
   if (x < g.w && y < g.h) {
-    const float2 a = chib[(int64_t)y * g.pitch + x];
+    const float2 a = chib[plane_of(g) + (int64_t)y * g.pitch + x];
     v[0] = (double)a.x * a.x + (double)a.y * a.y;
   }
   block_sum<1>(v, sh);
-  if (threadIdx.x == 0 && threadIdx.y == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = v[0];
+  if (threadIdx.x == 0 && threadIdx.y == 0) 
+    part[(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = v[0];
 }
 
-__global__ void k_adj_rhs(AdjGeom g, const float2* __restrict__ chib, float sigma,
-                          float2* __restrict__ B) {
+__global__ void k_adj_rhs(AdjGeom g, const AdjField* __restrict__ fields,
+                          const float2* __restrict__ chib, float2* __restrict__ B) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= g.w || y >= g.h) return;
-  const int64_t o = (int64_t)y * g.pitch + x;
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
   const float2 a = chib[o];
-  B[o] = make_float2(-sigma * a.x, -sigma * a.y);
+  const float sigma = fields[blockIdx.z].sigma;
+  B[o] = fields[blockIdx.z].active ? make_float2(-sigma * a.x, -sigma * a.y)
+                                   : make_float2(0.f, 0.f);
 }
 
-__global__ void k_adj_pass_a(AdjGeom g, AdjScalars sc, AdjOuter p) {
+__global__ void k_adj_pass_a(AdjGeom g, const AdjField* __restrict__ fields, AdjOuter p) {
   __shared__ double sh[4 * kBX * kBY / 32];
+  if (!fields[blockIdx.z].active) return;
+  const AdjScalars sc = fields[blockIdx.z].sc;
+  const float inv_sigma = 1.0f / fields[blockIdx.z].sigma;
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   double part[4] = {0.0, 0.0, 0.0, 0.0};
   if (x < g.w && y < g.h) {
-    const int64_t o = (int64_t)y * g.pitch + x;
+    const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
     const bool hx = x + 1 < g.w, hy = y + 1 < g.h;
     const float2 z = make_float2(0.f, 0.f);
     const float2 c = car(g, y, x);
     const float2 cr = hx ? car(g, y, x + 1) : z;
     const float2 cd = hy ? car(g, y + 1, x) : z;
     const float Sv = p.S[o], Sr = hx ? p.S[o + 1] : 0.f, Sd = hy ? p.S[o + g.pitch] : 0.f;
-    const float2 l0 = cmulf(p.lam[o], p.inv_sigma);
-    const float2 lr = hx ? cmulf(p.lam[o + 1], p.inv_sigma) : z;
-    const float2 ld = hy ? cmulf(p.lam[o + g.pitch], p.inv_sigma) : z;
+    const float2 l0 = cmulf(p.lam[o], inv_sigma);
+    const float2 lr = hx ? cmulf(p.lam[o + 1], inv_sigma) : z;
+    const float2 ld = hy ? cmulf(p.lam[o + g.pitch], inv_sigma) : z;
     const float r0 = re_mul(l0, c), rr = re_mul(lr, cr), rd = re_mul(ld, cd);
     const float dxr = hx ? rr - r0 : 0.f, dyr = hy ? rd - r0 : 0.f;
     const float2 a0 = p.chi1[o], ar = hx ? p.chi1[o + 1] : z, ad = hy ? p.chi1[o + g.pitch] : z;
@@ -157,30 +168,35 @@ __global__ void k_adj_pass_a(AdjGeom g, AdjScalars sc, AdjOuter p) {
   }
   block_sum<4>(part, sh);
   if (threadIdx.x == 0 && threadIdx.y == 0) {
-    double* dst = p.partials + 4 * (int64_t)(blockIdx.y * gridDim.x + blockIdx.x);
+    double* dst = p.partials +
+                  4 * (int64_t)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
 #pragma unroll
     for (int i = 0; i < 4; ++i) dst[i] = part[i];
   }
 }
 
-// acc[i] += sum_b part[4 b + i], b in order (one CTA)
-__global__ void k_adj_reduce(const double* __restrict__ part, int nb, int stride,
-                             double* __restrict__ acc) {
+// acc[i] += sum_b part[4 b + i], b in order (one CTA per field)
+__global__ void k_adj_reduce(const AdjField* __restrict__ fields, const double* __restrict__ part,
+                             int nb, double* __restrict__ acc) {
   __shared__ double sh[4 * 256 / 32];
+  if (!fields[blockIdx.x].active) return;
+  part += (int64_t)4 * nb * blockIdx.x;
+  acc += 4 * blockIdx.x;
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < nb; b += blockDim.x)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] += part[(int64_t)stride * b + i];
+    for (int i = 0; i < 4; ++i) v[i] += part[4LL * b + i];
   block_sum<4>(v, sh);
   if (threadIdx.x == 0)
-    for (int i = 0; i < 4 && i < stride; ++i) acc[i] += v[i];
+    for (int i = 0; i < 4; ++i) acc[i] += v[i];
 }
 
-__global__ void k_adj_pass_b(AdjGeom g, AdjOuter p, float* __restrict__ sbar,
-                             float2* __restrict__ chib) {
+__global__ void k_adj_pass_b(AdjGeom g, const AdjField* __restrict__ fields, AdjOuter p,
+                             float* __restrict__ sbar, float2* __restrict__ chib) {
+  if (!fields[blockIdx.z].active) return;
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= g.w || y >= g.h) return;
-  const int64_t o = (int64_t)y * g.pitch + x;
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
   const float2 z = make_float2(0.f, 0.f);
   // DxT / DyT of the interleaved planes, component by component
   const float2 pl = x > 0 ? p.P[o - 1] : z, pc = x < g.w - 1 ? p.P[o] : z;
@@ -201,7 +217,7 @@ __global__ void k_adj_pass_b(AdjGeom g, AdjOuter p, float* __restrict__ sbar,
 __global__ void k_ai_edges(AdjGeom g, AdjInit a) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= g.w || y >= g.h) return;
-  const int64_t o = (int64_t)y * g.pitch + x;
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
   const bool hx = x + 1 < g.w, hy = y + 1 < g.h;
   const float2 c = car(g, y, x);
   const float S0 = a.S[o];
@@ -224,9 +240,9 @@ __global__ void k_ai_box_v(AdjGeom g, const float2* __restrict__ in, float2* __r
   float2 s = make_float2(0.f, 0.f);
   for (int k = -3; k <= 3; ++k) {
     const int yy = y + k;
-    if (yy >= 0 && yy < g.h) s = cadd(s, in[(int64_t)yy * g.pitch + x]);
+    if (yy >= 0 && yy < g.h) s = cadd(s, in[plane_of(g) + (int64_t)yy * g.pitch + x]);
   }
-  out[(int64_t)y * g.pitch + x] = cmulf(s, 1.f / 7.f);
+  out[plane_of(g) + (int64_t)y * g.pitch + x] = cmulf(s, 1.f / 7.f);
 }
 __global__ void k_ai_box_h(AdjGeom g, const float2* __restrict__ in, float2* __restrict__ out) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
@@ -234,16 +250,16 @@ __global__ void k_ai_box_h(AdjGeom g, const float2* __restrict__ in, float2* __r
   float2 s = make_float2(0.f, 0.f);
   for (int k = -3; k <= 3; ++k) {
     const int xx = x + k;
-    if (xx >= 0 && xx < g.w) s = cadd(s, in[(int64_t)y * g.pitch + xx]);
+    if (xx >= 0 && xx < g.w) s = cadd(s, in[plane_of(g) + (int64_t)y * g.pitch + xx]);
   }
-  out[(int64_t)y * g.pitch + x] = cmulf(s, 1.f / 7.f);
+  out[plane_of(g) + (int64_t)y * g.pitch + x] = cmulf(s, 1.f / 7.f);
 }
 
 // blend adjoint: chi0 = (chi1 w1 + chi2 w2) / (w1 + w2), w = 1 / (E + 0.5)
 __global__ void k_ai_blend(AdjGeom g, AdjInit a) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= g.w || y >= g.h) return;
-  const int64_t o = (int64_t)y * g.pitch + x;
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
   const float2 E = a.a[o];
   const float w1 = 1.f / (E.x + 0.5f), w2 = 1.f / (E.y + 0.5f);
   const float ws = w1 + w2;
@@ -265,13 +281,13 @@ __global__ void k_ai_edges_adjoint(AdjGeom g, AdjInit a, const float2* __restric
                                    float* __restrict__ sbar) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= g.w || y >= g.h) return;
-  const int64_t o = (int64_t)y * g.pitch + x;
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
   const float2 c = car(g, y, x);
   float ys[2];
   for (int v = 0; v < 2; ++v) {
     const float2* chi = v == 0 ? a.chi1 : a.chi2;
     auto yv = [&](int yy, int xx) {
-      const int64_t oo = (int64_t)yy * g.pitch + xx;
+      const int64_t oo = plane_of(g) + (int64_t)yy * g.pitch + xx;
       return a.S[oo] - re_mul(chi[oo], car(g, yy, xx));
     };
     auto ab = [&](int64_t oo) { const float2 t = abar[oo]; return v == 0 ? t.x : t.y; };
@@ -285,74 +301,82 @@ __global__ void k_ai_edges_adjoint(AdjGeom g, AdjInit a, const float2* __restric
   }
   sbar[o] += ys[0] + ys[1];
   const int64_t plane = (int64_t)g.hp * g.pitch;
-  const int64_t oi = (int64_t)(y + g.pad) * g.pitch + x;
+  const int64_t oi = 2 * plane * blockIdx.z + (int64_t)(y + g.pad) * g.pitch + x;
   const float2 b1 = a.cb1[o], b2 = a.cb2[o];
   a.adj_in[oi] = make_float2(b1.x - ys[0] * c.x, b1.y + ys[0] * c.y);
   a.adj_in[plane + oi] = make_float2(b2.x - ys[1] * c.x, b2.y + ys[1] * c.y);
 }
 
-__device__ __forceinline__ int mirror101(int y, int h) {
-  if (h <= 1) return 0;
-  const int period = 2 * h - 2;
-  y = ((y % period) + period) % period;
-  return y < h ? y : period - y;
-}
-
-// one thread per column: sum the padded rows onto their mirror sources
+// Sum the padded rows onto their mirror sources, one thread per sample. The
+// pad is shorter than the plane (pad <= h - 1), so row y takes at most three
+// padded rows -- its images in the top pad, the plane and the bottom pad --
+// and adds them in that order. (One thread a column, walking all rows, took
+// 217 us for an NTSC field: six CTAs, and a serial chain of 300 loads.)
 __global__ void k_ai_fold(AdjGeom g, const float2* __restrict__ u, float* __restrict__ sbar) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= g.w) return;
+  const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
+  if (x >= g.w || y >= g.h) return;
   const int64_t plane = (int64_t)g.hp * g.pitch;
-  for (int r = 0; r < g.hp; ++r) {
-    const int sy = mirror101(r - g.pad, g.h);
-    const int64_t oi = (int64_t)r * g.pitch + x;
-    const float2 v = cadd(u[oi], u[plane + oi]);
-    sbar[(int64_t)sy * g.pitch + x] += re_mul(v, car(g, sy, x));
-  }
+  u += 2 * plane * blockIdx.z;
+  const float2 c = car(g, y, x);
+  const int64_t o = plane_of(g) + (int64_t)y * g.pitch + x;
+  float s = sbar[o];
+  auto add = [&](int row) {
+    const int64_t oi = (int64_t)(row + g.pad) * g.pitch + x;
+    s += re_mul(cadd(u[oi], u[plane + oi]), c);
+  };
+  const int below = 2 * (g.h - 1) - y;
+  if (y > 0 && y <= g.pad) add(-y);
+  add(y);
+  if (below > y && below < g.h + g.pad) add(below);
+  sbar[o] = s;
 }
 
-__global__ void k_adj_samples(AdjGeom g, const float* __restrict__ sbar, float inv_cpi, int fh,
-                              int fw, int fal, int a0, float* __restrict__ out) {
+__global__ void k_adj_samples(AdjGeom g, const AdjField* __restrict__ fields,
+                              const float* __restrict__ sbar, int fh, int fw, int fal, int a0,
+                              float* __restrict__ out) {
   const int x = blockIdx.x * kBX + threadIdx.x, y = blockIdx.y * kBY + threadIdx.y;
   if (x >= fw || y >= fh) return;
   const int ay = y - fal, ax = x - a0;
   float v = 0.f;
-  if (ay >= 0 && ay < g.h && ax >= 0 && ax < g.w) v = sbar[(int64_t)ay * g.pitch + ax] * inv_cpi;
-  out[(int64_t)y * fw + x] = v;
+  if (ay >= 0 && ay < g.h && ax >= 0 && ax < g.w) 
+    v = sbar[plane_of(g) + (int64_t)ay * g.pitch + ax] * fields[blockIdx.z].inv_cpi;
+  out[((int64_t)blockIdx.z * fh + y) * fw + x] = v;
 }
 
-dim3 grid_of(int w, int h) { return dim3((w + kBX - 1) / kBX, (h + kBY - 1) / kBY); }
+dim3 grid_of(int w, int h, int n) {
+  return dim3((w + kBX - 1) / kBX, (h + kBY - 1) / kBY, n);
+}
 
 }  // namespace
 
 int adj_blocks(const AdjGeom& g) {
-  const dim3 gr = grid_of(g.w, g.h);
+  const dim3 gr = grid_of(g.w, g.h, 1);
   return (int)(gr.x * gr.y);
 }
 
 void launch_adj_output(const AdjGeom& g, const float* ybar, float* sbar, float2* chibar,
                        cudaStream_t st) {
-  k_adj_output<<<grid_of(g.w, g.h), dim3(kBX, kBY), 0, st>>>(g, ybar, sbar, chibar);
+  k_adj_output<<<grid_of(g.w, g.h, g.n), dim3(kBX, kBY), 0, st>>>(g, ybar, sbar, chibar);
 }
 
 void launch_adj_norm(const AdjGeom& g, const float2* chibar, double* partials, cudaStream_t st) {
-  k_adj_norm<<<grid_of(g.w, g.h), dim3(kBX, kBY), 0, st>>>(g, chibar, partials);
+  k_adj_norm<<<grid_of(g.w, g.h, g.n), dim3(kBX, kBY), 0, st>>>(g, chibar, partials);
 }
 
-void launch_adj_rhs(const AdjGeom& g, const float2* chibar, float sigma, float2* B,
+void launch_adj_rhs(const AdjGeom& g, const AdjField* fields, const float2* chibar, float2* B,
                     cudaStream_t st) {
-  k_adj_rhs<<<grid_of(g.w, g.h), dim3(kBX, kBY), 0, st>>>(g, chibar, sigma, B);
+  k_adj_rhs<<<grid_of(g.w, g.h, g.n), dim3(kBX, kBY), 0, st>>>(g, fields, chibar, B);
 }
 
-void launch_adj_outer(const AdjGeom& g, const AdjScalars& sc, const AdjOuter& o, double* acc,
+void launch_adj_outer(const AdjGeom& g, const AdjField* fields, const AdjOuter& o, double* acc,
                       float* sbar, float2* chibar, cudaStream_t st) {
-  k_adj_pass_a<<<grid_of(g.w, g.h), dim3(kBX, kBY), 0, st>>>(g, sc, o);
-  k_adj_reduce<<<1, 256, 0, st>>>(o.partials, adj_blocks(g), 4, acc);
-  k_adj_pass_b<<<grid_of(g.w, g.h), dim3(kBX, kBY), 0, st>>>(g, o, sbar, chibar);
+  k_adj_pass_a<<<grid_of(g.w, g.h, g.n), dim3(kBX, kBY), 0, st>>>(g, fields, o);
+  k_adj_reduce<<<g.n, 256, 0, st>>>(fields, o.partials, adj_blocks(g), acc);
+  k_adj_pass_b<<<grid_of(g.w, g.h, g.n), dim3(kBX, kBY), 0, st>>>(g, fields, o, sbar, chibar);
 }
 
 void launch_adj_init_pointwise(const AdjGeom& g, const AdjInit& a, float* sbar, cudaStream_t st) {
-  const dim3 gr = grid_of(g.w, g.h), bl(kBX, kBY);
+  const dim3 gr = grid_of(g.w, g.h, g.n), bl(kBX, kBY);
   k_ai_edges<<<gr, bl, 0, st>>>(g, a);
   k_ai_box_v<<<gr, bl, 0, st>>>(g, a.a, a.tmp);
   k_ai_box_h<<<gr, bl, 0, st>>>(g, a.tmp, a.a);          // a -> E
@@ -363,13 +387,13 @@ void launch_adj_init_pointwise(const AdjGeom& g, const AdjInit& a, float* sbar, 
 }
 
 void launch_adj_fold(const AdjGeom& g, const float2* adj_out, float* sbar, cudaStream_t st) {
-  k_ai_fold<<<(g.w + 127) / 128, 128, 0, st>>>(g, adj_out, sbar);
+  k_ai_fold<<<grid_of(g.w, g.h, g.n), dim3(kBX, kBY), 0, st>>>(g, adj_out, sbar);
 }
 
-void launch_adj_samples(const AdjGeom& g, const float* sbar, float inv_cpi, int fh, int fw,
-                        int fal, int a0, float* samples_bar, cudaStream_t st) {
-  k_adj_samples<<<grid_of(fw, fh), dim3(kBX, kBY), 0, st>>>(g, sbar, inv_cpi, fh, fw, fal, a0,
-                                                           samples_bar);
+void launch_adj_samples(const AdjGeom& g, const AdjField* fields, const float* sbar, int fh,
+                        int fw, int fal, int a0, float* samples_bar, cudaStream_t st) {
+  k_adj_samples<<<grid_of(fw, fh, g.n), dim3(kBX, kBY), 0, st>>>(g, fields, sbar, fh, fw, fal, a0,
+                                                                samples_bar);
 }
 
 }  // namespace hvdg

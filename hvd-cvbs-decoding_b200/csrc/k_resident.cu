@@ -41,6 +41,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <functional>
+#include <vector>
 
 #include "hvdg_common.cuh"
 #include "k_solver.h"
@@ -1129,10 +1131,10 @@ ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag,
   while (max_rows > 0 && (nbr ? Smem<true>::bytes(max_rows) : Smem<false>::bytes(max_rows)) > 232448)
     --max_rows;
   double best_t = 0.0;
+  std::vector<double> cost(n), load;
   for (int g = 1; g <= std::min(n, sm_count); ++g) {
     const int c = std::min(sm_count / g, kMaxCtas);
     int rows = 0;
-    double total = 0.0, longest = 0.0;
     bool fits = true;
     for (int i = 0; i < n && fits; ++i) {
       const int ns = (shapes[i].w + kStrip - 1) / kStrip;
@@ -1147,12 +1149,18 @@ ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag,
       // a sweep costs its exchange plus its rows (us, measured: 4.1 at 21 rows, 5.4 at
       // 61, 6.6 at 73, 8.6 at 97, where g and q of seven rows fill the registers)
       const double sweep = 3.4 + 0.033 * tr + (tr > 80 ? 2.0 : 0.0);
-      const double t = shapes[i].n_outer * (shapes[i].n_inner + 3.0) * sweep + 5.0;
-      total += t;
-      longest = std::max(longest, t);
+      cost[i] = shapes[i].n_outer * (shapes[i].n_inner + 3.0) * sweep + 5.0;
     }
     if (!fits) break;
-    const double t = std::max(total / g, longest);
+    // the gangs take the fields heaviest first, each the next when it is free
+    std::sort(cost.begin(), cost.end(), [](double x, double y) { return x > y; });
+    load.assign(g, 0.0);
+    for (double t : cost) {
+      std::pop_heap(load.begin(), load.end(), std::greater<double>());
+      load.back() += t;
+      std::push_heap(load.begin(), load.end(), std::greater<double>());
+    }
+    const double t = *std::max_element(load.begin(), load.end());
     if (best.gangs == 0 || t < best_t) {
       best_t = t;
       best.gangs = g;

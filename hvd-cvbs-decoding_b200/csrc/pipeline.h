@@ -360,10 +360,11 @@ hvdg_status lockin_one(hvdg_ctx* ctx, const float* field_ire, const hvdg_geometr
 hvdg_status estimate_motion_sad(hvdg_ctx* ctx, const float* y_ref, const float* y_cur, int h,
                                 int w, int block, int range, float* dy, float* dx,
                                 float* confidence);
-hvdg_status decode_adjoint_field(hvdg_ctx* ctx, const hvdg_field_in& fi, const hvdg_config& cfg,
-                                 const float* y_bar, const float* chi_bar, float* samples_bar,
-                                 double* scalar_bar, int adj_iters, hvdg_field_out* out,
-                                 hvdg_diag* diag);
+hvdg_status decode_adjoint_fields(hvdg_ctx* ctx, const hvdg_field_in* fields, int n,
+                                  const hvdg_config& cfg, const float* const* y_bar,
+                                  const float* const* chi_bar, float* const* samples_bar,
+                                  double* scalar_bar, int adj_iters, hvdg_field_out* out,
+                                  hvdg_diag* diag);
 hvdg_status decode_woven_frames(hvdg_ctx* ctx, const int16_t* const* chroma,
                                 const int16_t* const* luma, int n, const hvdg_frame_params* fp,
                                 const hvdg_config* cfg, hvdg_yc_frame* out, hvdg_diag* diag,
