@@ -6,9 +6,10 @@
 // streaming kernel moves ~82 B of HBM or L2 per pixel in every CG iteration
 // and passes the phases of a lone field through a work queue; here a gang of
 // CTAs takes a whole field, each CTA keeps one tile of it (a 64-column strip
-// x up to 97 rows) for the entire solve -- g and q in registers, d, its luma
-// part, chi and the weights in shared memory -- and an iteration exchanges
-// only the tile edges' q and the CTA's partial sums.
+// x up to 112 rows) for the entire solve -- g, q and chi, which only their own
+// thread touches, in tensor memory; d, its luma part and the weights, which
+// neighbours read, in shared memory -- and an iteration exchanges only the
+// tile edges' q and the CTA's partial sums.
 //
 //  * Exchange: every word another CTA needs is published as a 16-byte slot
 //    {8 bytes of data, 8 bytes of tag} by one 128-bit store and polled by one
@@ -54,7 +55,7 @@ namespace {
 
 constexpr int kRT = 512;             // threads per CTA
 constexpr int kRW = kRT / 32;        // warps
-constexpr int kMaxRows = 97;         // tile rows that fit in shared memory
+constexpr int kMaxRows = 112;        // tile rows: seven per warp
 constexpr int kSideCap = 112;        // side slots per column (>= kMaxRows, multiple of 16)
 constexpr int kOutSlots = 2 * kStrip + 2 * kSideCap;
 constexpr int kSets = 3;             // edge slot sets
@@ -154,14 +155,14 @@ struct ResidentArgs {
 //    strip (luma part, horizontal weights, u); blocks 0 and rows + 1 are the
 //    rows above and below the tile.
 //  * W block r holds the weights (wx, wy, wcx, wcy) of each lane's even and odd
-//    pixel, chi, the line phasor (sw Lx, sw Ly, Lx, Ly) with sw the V-switch
+//    pixel, the line phasor (sw Lx, sw Ly, Lx, Ly) with sw the V-switch
 //    sense, and (kNbr) the neighbour data term.
 constexpr uint32_t kUB = 800;
 constexpr uint32_t kUR = 512, kY = 520, kYR = 776, kYL = 780, kWL = 784, kUL = 792;
-constexpr uint32_t kWb = 512, kChi = 1024, kLn = 1536, kM = 1552;
+constexpr uint32_t kWb = 512, kLn = 1024, kM = 1040;
 template <bool kNbr>
 struct Smem {
-  static constexpr uint32_t kWB = kNbr ? 2320 : 1552;
+  static constexpr uint32_t kWB = kNbr ? 1808 : 1040;
   uint32_t u, w, wtop;  // wtop: 64 x (wy, wcy) of the row above the tile
   double* part;         // kNV x warps
   double* res;          // kNV x collecting warps
@@ -261,6 +262,39 @@ __device__ __forceinline__ bool poll_slot(const Slot* p, unsigned long long tag,
     if (hi == tag) return true;
     if (++n > limit) return false;
   }
+}
+
+// Tensor memory as a second register file: what a thread alone reads and writes
+// -- g, q and chi of its two pixels in each row, four words each -- moved by
+// one instruction per row and waited for where it is used. With g and q in
+// registers (56 of 128 at seven rows) and chi in shared memory the sweep
+// spilled, and took 5.4 us at 61 rows, 7.5 at 81 and 8.6 at 97; this takes 4.8,
+// 5.6 and 6.2, and the shared memory freed holds 112 rows instead of 97.
+constexpr uint32_t kTg = 0, kTq = 4, kTc = 8, kTRow = 12;
+__device__ __forceinline__ void tmem_st4(uint32_t a, float2 u, float2 v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a),
+               "r"(__float_as_uint(u.x)), "r"(__float_as_uint(u.y)), "r"(__float_as_uint(v.x)),
+               "r"(__float_as_uint(v.y))
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t a, float2& u, float2& v) {
+  uint32_t r0, r1, r2, r3;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(a)
+               : "memory");
+  u = make_float2(__uint_as_float(r0), __uint_as_float(r1));
+  v = make_float2(__uint_as_float(r2), __uint_as_float(r3));
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// the values of a load are there only after the wait
+__device__ __forceinline__ void tmem_arrived(float2& u, float2& v) {
+  asm volatile("" : "+f"(u.x), "+f"(u.y), "+f"(v.x), "+f"(v.y)::"memory");
 }
 
 // This warp's rows: its first row's U and W blocks, and this lane's places in
@@ -453,8 +487,22 @@ __global__ void __launch_bounds__(kRT, 1)
                         reinterpret_cast<Slot*>(xb + (edge_bytes() + red_bytes()) * n_cta) +
                         R.gangs) + gang * R.ctas;
   const float2 z = make_float2(0.f, 0.f);
+  // tensor memory: a warp's lane quarter is its number modulo 4, the four warps
+  // of a quarter follow one another in columns, a row takes kTRow of them
+  constexpr uint32_t kNeed = NR * kTRow * (kRW / 4);
+  constexpr uint32_t kCols = kNeed <= 64 ? 64 : kNeed <= 128 ? 128 : kNeed <= 256 ? 256 : 512;
+  static_assert(kNeed <= 512, "columns of the SM's tensor memory");
+  if (wid == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(M.word + 3)),
+                 "r"(kCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
   if (tid == 0) M.word[0] = 0;
   __syncthreads();
+  const uint32_t tbase = (uint32_t)M.word[3];
+  const uint32_t tm = tbase + ((uint32_t)(wid & 3) << 21) + (uint32_t)(wid >> 2) * (NR * kTRow);
   int prev_parts = 0;  // CTAs of the gang's previous field (first CTA only)
   for (int ord = 0;; ++ord) {
     int idx = gang;
@@ -611,7 +659,6 @@ __global__ void __launch_bounds__(kRT, 1)
       }
     }
 
-    float2 ga[NR], gb[NR], qa[NR], qb[NR];
     const float m2h = 2.f * mu_h, m2v = 2.f * mu_v;
     // zero everything the stencil reads outside the field; line phasors; the
     // field's chi from its plane
@@ -632,8 +679,9 @@ __global__ void __launch_bounds__(kRT, 1)
           A.X[0] + base + (int64_t)(t.y0 + t.rb + i) * pitch + t.xa));
       if (!t.va) v.x = v.y = 0.f;
       if (!t.vb) v.z = v.w = 0.f;
-      sts4(rw.wl + i * WB + kChi, v);
+      tmem_st4(tm + kTRow * i + kTc, make_float2(v.x, v.y), make_float2(v.z, v.w));
     }
+    tmem_wait_st();
     __syncthreads();
     const unsigned long long tag_hi = (unsigned long long)(ord + 1) << 32;
     unsigned ex = 0;  // exchanges of this field so far
@@ -650,16 +698,17 @@ __global__ void __launch_bounds__(kRT, 1)
       {
         Slot* out = reinterpret_cast<Slot*>(xb + my_edges + set * kSetBytes);
         const unsigned long long tag = tag_hi | ex;
-#pragma unroll
-        for (int i = 0; i < NR; ++i) {
-          if (i >= t.nrow) break;
-          const float4 x4 = lds4(rw.wl + i * WB + kChi);
-          float2 xa = make_float2(x4.x, x4.y), xb2 = make_float2(x4.z, x4.w);
+#pragma unroll 1
+        for (int i = 0; i < t.nrow; ++i) {
+          float2 xa, xb2;
+          tmem_ld4(tm + kTRow * i + kTc, xa, xb2);
+          tmem_wait_ld();
+          tmem_arrived(xa, xb2);
           if (pending) {
             const float4 d4 = lds4(rw.ul + i * kUB);
             xa = cadd(xa, cscale(make_float2(d4.x, d4.y), alpha));
             xb2 = cadd(xb2, cscale(make_float2(d4.z, d4.w), alpha));
-            sts4(rw.wl + i * WB + kChi, make_float4(xa.x, xa.y, xb2.x, xb2.y));
+            tmem_st4(tm + kTRow * i + kTc, xa, xb2);
           }
           const float4 L = lds4(rw.w + i * WB + kLn);
           const float2 s2 = __ldcg(reinterpret_cast<const float2*>(
@@ -679,6 +728,7 @@ __global__ void __launch_bounds__(kRT, 1)
         }
       }
       pending = 0;
+      tmem_wait_st();
       __syncthreads();
       // ---- weights (lagged diffusivity), neighbour data term ----
       ++ex;
@@ -828,8 +878,7 @@ __global__ void __launch_bounds__(kRT, 1)
           }
           if (!t.va) oa = z;
           if (!t.vb) ob = z;
-          ga[i] = oa;
-          gb[i] = ob;
+          tmem_st4(tm + kTRow * i + kTg, oa, ob);
           pgg0 += (double)cnorm(oa) + (double)cnorm(ob);
           publish_row(t, out, lane, i, tag, oa, ob);
         }
@@ -839,6 +888,7 @@ __global__ void __launch_bounds__(kRT, 1)
           hg = unpack2(lo);
           hd = make_float2(-hg.x, -hg.y);
         }
+        tmem_wait_st();
       }
       __syncthreads();
       bad = M.word[0] != 0;
@@ -851,20 +901,30 @@ __global__ void __launch_bounds__(kRT, 1)
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
           if (i >= t.nrow) break;
-          float2 ua, ub;
+          float2 ua, ub, gka, gkb;
+          tmem_ld4(tm + kTRow * i + kTg, gka, gkb);
           if (first) {
-            ua = make_float2(-ga[i].x, -ga[i].y);
-            ub = make_float2(-gb[i].x, -gb[i].y);
+            tmem_wait_ld();
+            tmem_arrived(gka, gkb);
+            ua = make_float2(-gka.x, -gka.y);
+            ub = make_float2(-gkb.x, -gkb.y);
           } else {
-            const float4 d4 = lds4(rw.ul + i * kUB), x4 = lds4(rw.wl + i * WB + kChi);
+            float2 qka, qkb, xa, xb2;
+            tmem_ld4(tm + kTRow * i + kTq, qka, qkb);
+            tmem_ld4(tm + kTRow * i + kTc, xa, xb2);
+            const float4 d4 = lds4(rw.ul + i * kUB);
             const float2 doa = make_float2(d4.x, d4.y), dob = make_float2(d4.z, d4.w);
-            ga[i] = cadd(ga[i], cscale(qa[i], alpha));
-            gb[i] = cadd(gb[i], cscale(qb[i], alpha));
-            const float2 xa = cadd(make_float2(x4.x, x4.y), cscale(doa, alpha));
-            const float2 xb2 = cadd(make_float2(x4.z, x4.w), cscale(dob, alpha));
-            sts4(rw.wl + i * WB + kChi, make_float4(xa.x, xa.y, xb2.x, xb2.y));
-            ua = cadd(make_float2(-ga[i].x, -ga[i].y), cscale(doa, beta));
-            ub = cadd(make_float2(-gb[i].x, -gb[i].y), cscale(dob, beta));
+            tmem_wait_ld();
+            tmem_arrived(gka, gkb);
+            tmem_arrived(qka, qkb);
+            tmem_arrived(xa, xb2);
+            tmem_st4(tm + kTRow * i + kTc, cadd(xa, cscale(doa, alpha)),
+                     cadd(xb2, cscale(dob, alpha)));
+            gka = cadd(gka, cscale(qka, alpha));
+            gkb = cadd(gkb, cscale(qkb, alpha));
+            tmem_st4(tm + kTRow * i + kTg, gka, gkb);
+            ua = cadd(make_float2(-gka.x, -gka.y), cscale(doa, beta));
+            ub = cadd(make_float2(-gkb.x, -gkb.y), cscale(dob, beta));
           }
           const float4 L = lds4(rw.w + i * WB + kLn);
           sts4(rw.ul + i * kUB, make_float4(ua.x, ua.y, ub.x, ub.y));
@@ -875,6 +935,7 @@ __global__ void __launch_bounds__(kRT, 1)
           sts2(hu, hd);
           sts1(hyp, -re_rn(hd, hc));
         }
+        tmem_wait_st();
         __syncthreads();
         // ---- q = A d, the curvature and the inner products ----
         ++ex;
@@ -891,6 +952,8 @@ __global__ void __launch_bounds__(kRT, 1)
             if (i >= t.nrow) break;
             const float4 L = lds4(rw.w + i * WB + kLn);
             const float2 cua = c.ua, cub = c.ub;
+            float2 gka, gkb;
+            tmem_ld4(tm + kTRow * i + kTg, gka, gkb);
             RowDiff d;
             float2 oa, ob;
             stencil_row<true, kNbr>(rw, i, lane, car_rn(L, t.Pa), car_rn(L, t.Pb), m2h, m2v, c, d,
@@ -916,17 +979,18 @@ __global__ void __launch_bounds__(kRT, 1)
             rH += curv_sum(__fmaf_rn(d.ayb, d.dyyb, __fmul_rn(d.axb, d.dxyb)),
                            __fmul_rn(mu_h, d.wb.z), norm_xy(d.dxub), __fmul_rn(mu_v, d.wb.w),
                            norm_xy(d.dyub));
-            const float2 gka = ga[i], gkb = gb[i];
+            tmem_wait_ld();
+            tmem_arrived(gka, gkb);
             pv[0] += (double)rH;
             pv[1] += (double)(dot_yx(gka, cua) + dot_yx(gkb, cub));
             pv[2] += (double)(dot_yx(gka, oa) + dot_yx(gkb, ob));
             pv[3] += (double)(norm_yx(oa) + norm_yx(ob));
             pv[4] += (double)(norm_yx(gka) + norm_yx(gkb));
-            qa[i] = oa;
-            qb[i] = ob;
+            tmem_st4(tm + kTRow * i + kTq, oa, ob);
             publish_row(t, out, lane, i, tag, oa, ob);
           }
         }
+        tmem_wait_st();
         // ---- the CTA's sums ----
         {
           double v;
@@ -1042,8 +1106,10 @@ __global__ void __launch_bounds__(kRT, 1)
     for (int i = 0; i < t.nrow; ++i) {
       const int r = t.rb + i, y = t.y0 + r;
       const int64_t o = (int64_t)y * pitch + t.xa;
-      const float4 x4 = lds4(rw.wl + i * WB + kChi);
-      float2 xa = make_float2(x4.x, x4.y), xb2 = make_float2(x4.z, x4.w);
+      float2 xa, xb2;
+      tmem_ld4(tm + kTRow * i + kTc, xa, xb2);
+      tmem_wait_ld();
+      tmem_arrived(xa, xb2);
       if (pending) {
         const float4 d4 = lds4(rw.ul + i * kUB);
         xa = cadd(xa, cscale(make_float2(d4.x, d4.y), alpha));
@@ -1095,6 +1161,10 @@ __global__ void __launch_bounds__(kRT, 1)
     __syncthreads();
     if (tid == 0) st_release(done + cta, ord + 1);
   }
+  __syncthreads();
+  if (wid == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase),
+                 "r"(kCols));
 }
 
 template <int NR, bool kNbr>
@@ -1146,9 +1216,9 @@ ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag,
       const int tr = (shapes[i].h + nv - 1) / nv;
       rows = std::max(rows, tr);
       fits = tr <= max_rows;
-      // a sweep costs its exchange plus its rows (us, measured: 4.1 at 21 rows, 5.4 at
-      // 61, 6.6 at 73, 8.6 at 97, where g and q of seven rows fill the registers)
-      const double sweep = 3.4 + 0.033 * tr + (tr > 80 ? 2.0 : 0.0);
+      // a sweep costs its exchange plus its rows (us, measured: 3.5 at 25 rows, 4.1 at
+      // 41, 4.8 at 61, 5.6 at 81, 6.2 at 97)
+      const double sweep = 3.0 + 0.033 * tr;
       cost[i] = shapes[i].n_outer * (shapes[i].n_inner + 3.0) * sweep + 5.0;
     }
     if (!fits) break;

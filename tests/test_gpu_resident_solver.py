@@ -50,6 +50,7 @@ def _both(ctx, call):
     (1, 700, 33, 5, 0.0),
     (0, 0, 0, 7, 0.0),         # whole fields, more than the gangs
     (1, 0, 0, 4, 0.0),         # 97-row tiles
+    (0, 0, 110, 12, 0.0),      # seven rows a warp, the last one short
     (1, 129, 40, 1, 4.4340e6),  # a declared subcarrier: general phasors
 ])
 def test_planes_equal_streaming(std, w, lines, n, sub):
