@@ -149,6 +149,9 @@ void hvdg_destroy(hvdg_ctx* ctx) {
   for (auto& ev : ctx->ev) cudaEventDestroy(ev);
   if (ctx->ev_in) cudaEventDestroy(ctx->ev_in);
   if (ctx->ev_done) cudaEventDestroy(ctx->ev_done);
+  for (cudaEvent_t ev : ctx->frame_ev) cudaEventDestroy(ev);
+  if (ctx->h2d) cudaStreamDestroy(ctx->h2d);
+  if (ctx->d2h) cudaStreamDestroy(ctx->d2h);
   if (ctx->flags_host) cudaFreeHost(ctx->flags_host);
   if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
   cudaStreamDestroy(ctx->stream);

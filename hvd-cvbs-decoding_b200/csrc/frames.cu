@@ -439,10 +439,64 @@ hvdg_status detect_field_parity_frames(hvdg_ctx* ctx, const int16_t* const* fram
 // S and of the line phasors straight into the woven plane (crop rows and
 // line_step), holographic init on the woven plane (column length 2048),
 // then -- composite only -- aniso + IRLS / CG; re-weave and requantisation
-// (k_frame_out). On the host: the field-order vote and the copies.
+// (k_frame_out). On the host: the copies.
 // `chroma` frames are the composite frames (yc = false) or the C channel
 // (yc = true, with `luma` the Y channel passed through).
+//
+// The frames go through in chunks: their copies, on two streams of their own,
+// run beside the other chunks' kernels (the copies of 8 PAL Y/C frames take
+// 2.4 ms, their kernels 0.7 in one chunk; end to end 3.57 ms in one chunk,
+// 2.87 by twos, where the kernels' latency at small sizes makes 1.8 ms of
+// them; 3.25 one by one). A chunk is two frames where nothing is solved;
+// otherwise one or two rounds of the solver's gangs (8 NTSC frames: 2.85 ms
+// together, 2.45 by twos, 2.37 by fours). Planes that the streaming solver
+// takes stay together.
 // ---------------------------------------------------------------------------
+namespace {
+
+constexpr int kFrameChunks = 16;
+enum { kEvIn, kEvInit, kEvSolve, kEvSolved, kEvOut, kEvChunk };  // events of a chunk
+
+// The streams of a chunked call end with it, on every path.
+struct FrameStreams {
+  hvdg_ctx* ctx;
+  ~FrameStreams() {
+    cudaStreamSynchronize(ctx->h2d);
+    cudaStreamSynchronize(ctx->stream);
+    cudaStreamSynchronize(ctx->d2h);
+  }
+};
+
+hvdg_status frame_streams(hvdg_ctx* ctx, int chunks) {
+  cudaError_t e = cudaSuccess;
+  if (!ctx->h2d) e = cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking);
+  if (e == cudaSuccess && !ctx->d2h) e = cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking);
+  while (e == cudaSuccess && (int)ctx->frame_ev.size() < chunks * kEvChunk + 1) {
+    cudaEvent_t ev;
+    e = cudaEventCreate(&ev);
+    if (e == cudaSuccess) ctx->frame_ev.push_back(ev);
+  }
+  return e == cudaSuccess ? HVDG_OK : hvdg::cuda_fail(ctx, e, "frame streams");
+}
+
+int frame_chunk(hvdg_ctx* ctx, const hvdg_field_in* fi, int n, const hvdg_config* cfg,
+                const RunOpts& opt) {
+  int c = 2;
+  if (opt.do_solve) {
+    std::vector<int> order;
+    if (!resident_allowed(ctx)) return n;
+    const std::vector<ResidentGroup> g =
+        resident_groups(ctx, solve_shapes(fi, 2 * n, cfg, opt.weave_geom), false,
+                        cfg->diag_prior > 0.0f, &order);
+    if (g.empty()) return n;
+    c = g[0].plan.gangs * (n >= 4 * g[0].plan.gangs ? 2 : 1);
+  }
+  const int rounds = (n + c - 1) / c;
+  return c * ((rounds + kFrameChunks - 1) / kFrameChunks);
+}
+
+}  // namespace
+
 hvdg_status decode_woven_frames(hvdg_ctx* ctx, const int16_t* const* chroma,
                                 const int16_t* const* luma, int n, const hvdg_frame_params* fp,
                                 const hvdg_config* cfg, hvdg_yc_frame* out, hvdg_diag* diag,
@@ -515,148 +569,208 @@ hvdg_status decode_woven_frames(hvdg_ctx* ctx, const int16_t* const* chroma,
   const size_t o_vote = align_up(o_ov + sizeof(double) * npx * n, 256);
   const size_t o_arrive = align_up(o_vote + sizeof(int) * n, 256);
   const size_t o_part = align_up(o_arrive + sizeof(int) * n, 256);
-  const size_t xbytes = align_up(o_part + (device_vote ? sizeof(double) * 2 * vg.blocks * n : 0), 256);
-  Staged S;
-  st = stage_upload(ctx, fi.data(), 2 * n, cfg, opt, xbytes, S);
+  const size_t o_flags = align_up(o_part + (device_vote ? sizeof(double) * 2 * vg.blocks * n : 0), 256);
+  const size_t o_ctl = align_up(o_flags + sizeof(int) * 4 * n, 256);
+  const size_t o_amp = align_up(o_ctl + sizeof(FieldCtl) * n, 256);
+  const size_t xbytes = align_up(o_amp + sizeof(float) * 2, 256);
+  const int chunk = std::min(n, frame_chunk(ctx, fi.data(), n, cfg, opt));
+  const int n_chunks = (n + chunk - 1) / chunk;
+  st = frame_streams(ctx, n_chunks);
   if (st != HVDG_OK) return st;
-  const Batch& b = S.b;
-  const Layout& L = b.L;
+  FrameStreams streams{ctx};
   cudaStream_t s = ctx->stream;
-  char* X = at<char>(ctx, S.extra);
+  cudaEvent_t* const ev = ctx->frame_ev.data() + 1;
+  Staged S;
+  st = stage_upload(ctx, fi.data(), 2 * chunk, cfg, opt, xbytes, S);
+  if (st != HVDG_OK) return st;
+  char* const X = at<char>(ctx, S.extra);
   std::vector<int64_t> loff(fh);
   for (int y = 0; y < fh; ++y) loff[y] = frame_line_offset(P, y);
   cudaError_t e = cudaMemcpyAsync(X + o_lines, loff.data(), sizeof(int64_t) * fh,
                                   cudaMemcpyHostToDevice, s);
-  for (int t = 0; t < n && e == cudaSuccess; ++t) {
-    e = cudaMemcpyAsync(X + o_src + sizeof(int16_t) * stride * t, chroma[t], sizeof(int16_t) * need,
-                        cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && yc)
-      e = cudaMemcpyAsync(X + o_pass + sizeof(int16_t) * stride * t, luma[t],
-                          sizeof(int16_t) * need, cudaMemcpyHostToDevice, s);
-  }
+  // (a new arena is cleared on the context's stream)
+  if (e == cudaSuccess) e = cudaEventRecord(ev[-1], s);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->h2d, ev[-1], 0);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "H2D frames");
-  mark(ctx, 0);  // device time of the kernels: from the split to the re-weave
   const float cpi = (P.white_level - P.blanking_level) / 100.0f;
-  hvdg::FrameSplitArgs sp;
-  sp.frames = reinterpret_cast<const int16_t*>(X + o_src);
-  sp.frame_stride = stride;
-  sp.line_off = reinterpret_cast<const int64_t*>(X + o_lines);
-  sp.fw = fw;
-  sp.fh = fh;
-  sp.f1 = f1;
-  sp.center = yc ? P.chroma_dc : P.blanking_level;
-  sp.codes_per_ire = cpi;
-  sp.fields = at<float>(ctx, L.o_raw);
-  sp.field_stride = (b.pp.size() > 1 ? b.pp[1].raw_off - b.pp[0].raw_off : 0) / (int64_t)sizeof(float);
-  sp.order = split_order;
-  sp.vote = reinterpret_cast<const int*>(X + o_vote);
-  if (device_vote) {
-    hvdg::FrameVoteArgs va = vg;
-    va.frames = sp.frames;
-    va.frame_stride = stride;
-    va.line_off = sp.line_off;
-    va.vote = reinterpret_cast<int*>(X + o_vote);
-    va.arrive = reinterpret_cast<int*>(X + o_arrive);
-    va.partial = reinterpret_cast<double*>(X + o_part);
-    hvdg::launch_frame_vote(va, n, s);
-    S.launches += 1;
-  }
-  hvdg::launch_frame_split(sp, n, s);
-  S.launches += 1;
-  st = stage_prepare(ctx, S, opt);
-  if (st != HVDG_OK) return st;
-  hvdg::launch_burst_amplitude(at<hvdg::PrepDesc>(ctx, L.o_prep), 2 * n, at<float>(ctx, L.o_amp), s);
-  S.launches += 1;
-  if (opt.do_solve) {
-    hvdg::launch_aniso(at<FieldDesc>(ctx, L.o_fields), n, at<float2>(ctx, L.o_X0), s);
-    S.launches += 1;
-  }
-  mark(ctx, 2);
-  if (opt.do_solve) {
-    const hvdg::SolverArgs sa = solver_args(ctx, S);
-    e = launch_solve(ctx, S, sa, b.rg, false, opt.ctas_per_sm);
-    if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
-    S.launches += 1;
-  }
-  mark(ctx, 3);
-  const FieldPlan& p0 = b.fp[0];
-  hvdg::FrameOutArgs fo;
-  fo.Y = at<float>(ctx, L.o_Y);
-  fo.chi = at<float2>(ctx, L.o_X0);
-  fo.S = at<float>(ctx, L.o_S);
-  fo.plane_stride = n > 1 ? b.fp[1].px_off - p0.px_off : 0;
-  fo.pitch = p0.pitch;
-  fo.h = p0.h;
-  fo.w = p0.w;
-  fo.line_phasor = at<float4>(ctx, L.o_lineph);
-  fo.col_phasor = at<float2>(ctx, L.o_colph);
-  fo.amp = at<float>(ctx, L.o_amp);
-  fo.passthrough = reinterpret_cast<const int16_t*>(X + (yc ? o_pass : o_src));
-  fo.frame_stride = stride;
-  fo.line_off = reinterpret_cast<const int64_t*>(X + o_lines);
-  fo.fw = fw;
-  fo.fh = fh;
-  fo.f1 = f1;
-  fo.fal = g.first_active_field_line;
-  fo.a0 = P.active_video_start;
-  fo.blank = P.blanking_level;
-  fo.scale = cpi;
-  fo.chroma_gain = cfg->chroma_gain;
-  fo.nominal_burst = nominal_burst(g);
-  fo.acc = cfg->acc ? 1 : 0;
-  fo.yc = yc ? 1 : 0;
-  fo.mono = (!yc && cfg->monochrome) ? 1 : 0;
-  fo.luma = reinterpret_cast<int16_t*>(X + o_ol);
-  fo.chroma = reinterpret_cast<int16_t*>(X + o_oc);
-  fo.u = reinterpret_cast<double*>(X + o_ou);
-  fo.v = reinterpret_cast<double*>(X + o_ov);
-  hvdg::launch_frame_out(fo, n, s);
-  S.launches += 1;
-  mark(ctx, 4);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "frame kernels");
-  for (int t = 0; t < n && e == cudaSuccess; ++t) {
-    e = cudaMemcpyAsync(out[t].luma, fo.luma + npx * t, sizeof(int16_t) * npx,
-                        cudaMemcpyDeviceToHost, s);
+  // A chunk's planes go back once the next one's kernels are queued: a copy to
+  // pageable memory holds the host until it is done.
+  auto copy_back = [&](int k) {
+    cudaError_t r = cudaStreamWaitEvent(ctx->d2h, ev[k * kEvChunk + kEvOut], 0);
+    for (int t = k * chunk; t < std::min(n, (k + 1) * chunk); ++t) {
+      auto back = [&](void* dst, size_t off, size_t px) {
+        if (r == cudaSuccess)
+          r = cudaMemcpyAsync(dst, X + off + px * npx * t, px * npx, cudaMemcpyDeviceToHost,
+                              ctx->d2h);
+      };
+      back(out[t].luma, o_ol, sizeof(int16_t));
+      back(out[t].chroma, o_oc, sizeof(int16_t));
+      back(out[t].u_plane, o_ou, sizeof(double));
+      back(out[t].v_plane, o_ov, sizeof(double));
+    }
+    return r;
+  };
+  int launches = 0;
+  for (int k = 0; k < n_chunks; ++k) {
+    const int t0 = k * chunk, m = std::min(chunk, n - t0);
+    cudaEvent_t* const ek = ev + k * kEvChunk;
+    if (k > 0 && m != (int)S.b.fp.size()) {
+      S = Staged();
+      st = stage_upload(ctx, fi.data(), 2 * m, cfg, opt, 0, S);
+      if (st != HVDG_OK) return st;
+    } else if (k > 0) {
+      stage_reset(ctx, S);
+    }
+    const Batch& b = S.b;
+    const Layout& L = b.L;
+    const int16_t* const src = reinterpret_cast<const int16_t*>(X + o_src) + stride * t0;
+    const int16_t* const pass = reinterpret_cast<const int16_t*>(X + o_pass) + stride * t0;
+    for (int t = 0; t < m && e == cudaSuccess; ++t) {
+      e = cudaMemcpyAsync(const_cast<int16_t*>(src) + stride * t, chroma[t0 + t],
+                          sizeof(int16_t) * need, cudaMemcpyHostToDevice, ctx->h2d);
+      if (e == cudaSuccess && yc)
+        e = cudaMemcpyAsync(const_cast<int16_t*>(pass) + stride * t, luma[t0 + t],
+                            sizeof(int16_t) * need, cudaMemcpyHostToDevice, ctx->h2d);
+    }
+    // device time of the kernels: from the split to the re-weave
+    if (e == cudaSuccess) e = cudaEventRecord(ek[kEvIn], ctx->h2d);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ek[kEvIn], 0);
+    if (e == cudaSuccess) e = cudaEventRecord(ek[kEvIn], s);
+    if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "H2D frames");
+    hvdg::FrameSplitArgs sp;
+    sp.frames = src;
+    sp.frame_stride = stride;
+    sp.line_off = reinterpret_cast<const int64_t*>(X + o_lines);
+    sp.fw = fw;
+    sp.fh = fh;
+    sp.f1 = f1;
+    sp.center = yc ? P.chroma_dc : P.blanking_level;
+    sp.codes_per_ire = cpi;
+    sp.fields = at<float>(ctx, L.o_raw);
+    sp.field_stride = (b.pp.size() > 1 ? b.pp[1].raw_off - b.pp[0].raw_off : 0) / (int64_t)sizeof(float);
+    sp.order = split_order;
+    sp.vote = reinterpret_cast<const int*>(X + o_vote) + t0;
+    if (device_vote) {
+      hvdg::FrameVoteArgs va = vg;
+      va.frames = sp.frames;
+      va.frame_stride = stride;
+      va.line_off = sp.line_off;
+      va.vote = reinterpret_cast<int*>(X + o_vote) + t0;
+      va.arrive = reinterpret_cast<int*>(X + o_arrive) + t0;
+      va.partial = reinterpret_cast<double*>(X + o_part) + (int64_t)2 * vg.blocks * t0;
+      hvdg::launch_frame_vote(va, m, s);
+      launches += 1;
+    }
+    hvdg::launch_frame_split(sp, m, s);
+    launches += 1;
+    if (diag) cudaEventRecord(ek[kEvInit], s);
+    S.launches = 0;
+    st = stage_prepare(ctx, S, opt);
+    if (st != HVDG_OK) return st;
+    hvdg::launch_burst_amplitude(at<hvdg::PrepDesc>(ctx, L.o_prep), 2 * m, at<float>(ctx, L.o_amp), s);
+    launches += S.launches + 1;
+    if (opt.do_solve) {
+      hvdg::launch_aniso(at<FieldDesc>(ctx, L.o_fields), m, at<float2>(ctx, L.o_X0), s);
+      launches += 1;
+    }
+    if (diag) cudaEventRecord(ek[kEvSolve], s);
+    if (opt.do_solve) {
+      const hvdg::SolverArgs sa = solver_args(ctx, S);
+      e = launch_solve(ctx, S, sa, b.rg, false, opt.ctas_per_sm);
+      if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
+      launches += 1;
+    }
+    if (diag) cudaEventRecord(ek[kEvSolved], s);
+    const FieldPlan& p0 = b.fp[0];
+    hvdg::FrameOutArgs fo;
+    fo.Y = at<float>(ctx, L.o_Y);
+    fo.chi = at<float2>(ctx, L.o_X0);
+    fo.S = at<float>(ctx, L.o_S);
+    fo.plane_stride = m > 1 ? b.fp[1].px_off - p0.px_off : 0;
+    fo.pitch = p0.pitch;
+    fo.h = p0.h;
+    fo.w = p0.w;
+    fo.line_phasor = at<float4>(ctx, L.o_lineph);
+    fo.col_phasor = at<float2>(ctx, L.o_colph);
+    fo.amp = at<float>(ctx, L.o_amp);
+    fo.passthrough = yc ? pass : src;
+    fo.frame_stride = stride;
+    fo.line_off = reinterpret_cast<const int64_t*>(X + o_lines);
+    fo.fw = fw;
+    fo.fh = fh;
+    fo.f1 = f1;
+    fo.fal = g.first_active_field_line;
+    fo.a0 = P.active_video_start;
+    fo.blank = P.blanking_level;
+    fo.scale = cpi;
+    fo.chroma_gain = cfg->chroma_gain;
+    fo.nominal_burst = nominal_burst(g);
+    fo.acc = cfg->acc ? 1 : 0;
+    fo.yc = yc ? 1 : 0;
+    fo.mono = (!yc && cfg->monochrome) ? 1 : 0;
+    fo.luma = reinterpret_cast<int16_t*>(X + o_ol) + npx * t0;
+    fo.chroma = reinterpret_cast<int16_t*>(X + o_oc) + npx * t0;
+    fo.u = reinterpret_cast<double*>(X + o_ou) + npx * t0;
+    fo.v = reinterpret_cast<double*>(X + o_ov) + npx * t0;
+    hvdg::launch_frame_out(fo, m, s);
+    launches += 1;
+    // the chunk's control state: the next one resets it
+    e = cudaMemcpyAsync(X + o_flags + sizeof(int) * 4 * k, at<int>(ctx, L.o_flags), sizeof(int) * 4,
+                        cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(out[t].chroma, fo.chroma + npx * t, sizeof(int16_t) * npx,
-                          cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(out[t].u_plane, fo.u + npx * t, sizeof(double) * npx,
-                          cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(out[t].v_plane, fo.v + npx * t, sizeof(double) * npx,
-                          cudaMemcpyDeviceToHost, s);
+      e = cudaMemcpyAsync(X + o_ctl + sizeof(FieldCtl) * t0, at<FieldCtl>(ctx, L.o_ctl),
+                          sizeof(FieldCtl) * m, cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess && k == 0)
+      e = cudaMemcpyAsync(X + o_amp, at<float>(ctx, L.o_amp), sizeof(float) * 2,
+                          cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaEventRecord(ek[kEvOut], s);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "frame kernels");
+    if (k > 0) e = copy_back(k - 1);
+    if (e == cudaSuccess && k == n_chunks - 1) e = copy_back(k);
+    if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "D2H frames");
   }
-  if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "D2H frames");
-  int flags[4] = {0, 0, 0, 0};
+  std::vector<int> chunk_flags(4 * n_chunks);
   float amp01[2] = {0.f, 0.f};
   std::vector<FieldCtl> ctl(n);
-  e = cudaMemcpyAsync(flags, at<int>(ctx, L.o_flags), sizeof(flags), cudaMemcpyDeviceToHost, s);
+  e = cudaMemcpyAsync(chunk_flags.data(), X + o_flags, sizeof(int) * chunk_flags.size(),
+                      cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(amp01, at<float>(ctx, L.o_amp), sizeof(amp01), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(amp01, X + o_amp, sizeof(amp01), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && diag)
-    e = cudaMemcpyAsync(ctl.data(), at<FieldCtl>(ctx, L.o_ctl), sizeof(FieldCtl) * n,
-                        cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(ctl.data(), X + o_ctl, sizeof(FieldCtl) * n, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->d2h);
   if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "frame decode sync");
+  int flags[2] = {0, 0};
+  for (int k = 0; k < n_chunks; ++k)
+    for (int i = 0; i < 2; ++i) flags[i] |= chunk_flags[4 * k + i];
   if (diag) {
-    diag->ms_total = elapsed(ctx, 0, 4);
-    diag->ms_solver = elapsed(ctx, 2, 3);
-    diag->ms_init = elapsed(ctx, 1, 2);
+    auto between = [&](int k, int a, int b) {
+      float ms = 0.f;
+      if (cudaEventElapsedTime(&ms, ev[k * kEvChunk + a], ev[k * kEvChunk + b]) != cudaSuccess) {
+        cudaGetLastError();
+        ms = 0.f;
+      }
+      return ms;
+    };
+    for (int k = 0; k < n_chunks; ++k) {
+      diag->ms_total += between(k, kEvIn, kEvOut);
+      diag->ms_solver += between(k, kEvSolve, kEvSolved);
+      diag->ms_init += between(k, kEvInit, kEvSolve);
+    }
     float acc = 1.0f;
     if (cfg->acc) {
       const float m = 0.5f * (amp01[0] + amp01[1]);
       acc = std::min(std::max(nominal_burst(g) / std::max(m, 1.0f), 0.5f), 2.0f);
     }
     diag->acc_gain = acc;
-    for (int i = 0; i < n; ++i) {
-      if (opt.do_solve) diag->cg_iterations_run += ctl[i].cg_iters;
-      if (opt.do_solve) diag->solver_pixel_iters += (int64_t)ctl[i].cg_iters * b.fp[i].h * b.fp[i].w;
-      if (opt.do_solve)
-        diag->solver_pixel_outers += (int64_t)b.fields[i].n_outer * b.fp[i].h * b.fp[i].w;
+    for (int i = 0; i < n && opt.do_solve; ++i) {
+      diag->cg_iterations_run += ctl[i].cg_iters;
+      diag->solver_pixel_iters += (int64_t)ctl[i].cg_iters * 2 * lines * w;
+      diag->solver_pixel_outers += (int64_t)S.b.fields[0].n_outer * 2 * lines * w;
     }
-    diag->kernel_launches = S.launches;
+    diag->kernel_launches = launches;
   }
   if (flags[1]) {
     ctx->last_error = "non-finite input samples";

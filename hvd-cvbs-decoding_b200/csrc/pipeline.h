@@ -145,6 +145,9 @@ struct hvdg_ctx {
   // asynchronous device-resident decodes: ordering against the caller's
   // stream, completion, and the result of a call that awaits hvdg_wait
   cudaEvent_t ev_in = nullptr, ev_done = nullptr;
+  // the woven-frame calls' copies (created at the first one)
+  cudaStream_t h2d = nullptr, d2h = nullptr;
+  std::vector<cudaEvent_t> frame_ev;
   bool pending = false;           // a replay is in flight, hvdg_wait reads its flags
   bool settled = false;           // pending_status / pending_diag hold a finished call
   hvdg_status pending_status = HVDG_OK;
