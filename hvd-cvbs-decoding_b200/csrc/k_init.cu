@@ -815,91 +815,151 @@ __global__ void __launch_bounds__(kLongThreads) k_sym_cols_long(InitArgs a, int 
 }
 
 // ---- blend -----------------------------------------------------------------
-// Edge-energy blend (holographic_init.cpp:240-316). 32 x 32 output tile per
-// CTA; y_v on the tile + 4 halo (forward difference + box radius 3); the box
-// blur is zero-padded at the field border with constant 1/7 normalisation.
-constexpr int kBT = 32;
-constexpr int kBH = kBT + 8;  // y_v tile incl. halo [-3, +4]
-__global__ void __launch_bounds__(256) k_init_blend(InitArgs a) {
+// Edge-energy blend (holographic_init.cpp:240-316): per variant v the residual
+// luma y_v = S - Re[chi_v c], the edge energy e = |Dx y_v| + |Dy y_v| (forward,
+// zero on the last column / row), its 7 x 7 box mean E (vertical first,
+// zero-padded at the field border, constant 1/7), weights 1 / (E + 0.5).
+//
+// A warp walks down 64 columns, two to a lane, of which it outputs the middle
+// 56: the last row's y_v and the last seven rows' e stay in registers, a row's
+// box sums take their neighbours by shuffle, and the next row's loads are in
+// flight meanwhile. chi_v and S of the row that is output, four rows up, come
+// from the L1 again. @BLEND@
+constexpr int kBC = 56;  // columns of a warp's tile; its rows are a.blend_rows
+
+template <int NV>
+struct BlendRow {
+  float2 s;
+  float4 c[NV];
+  float4 L;
+};
+
+__device__ __forceinline__ float2 blend_car(float4 L, float2 P) {
+  const float x = __fmaf_rn(L.x, P.x, -__fmul_rn(L.y, P.y));
+  return make_float2(L.z < 0.f ? -x : x, __fmaf_rn(L.x, P.y, __fmul_rn(L.y, P.x)));
+}
+__device__ __forceinline__ float blend_luma(float S, float2 u, float2 c) {
+  return S - __fmaf_rn(u.x, c.x, -__fmul_rn(u.y, c.y));
+}
+
+template <int NV>
+__global__ void __launch_bounds__(32) k_init_blend(InitArgs a) {
   const int f_idx = a.btile_field[blockIdx.x];
-  const FieldDesc f = a.fields[f_idx];
+  const FieldDesc& f = a.fields[f_idx];
+  const int fw = f.w, fh = f.h, pitch = f.pitch;
   const int t = blockIdx.x - a.btile_first[f_idx];
-  const int ntx = (f.w + kBT - 1) / kBT;
-  const int ty0 = (t / ntx) * kBT, tx0 = (t % ntx) * kBT;
-  __shared__ float yv[kBH][kBH + 1];
-  __shared__ float ev[kBH][kBH + 1];
-  __shared__ float vb[kBT][kBH + 1];
-  __shared__ float wsum[kBT][kBT];
-  __shared__ float2 num[kBT][kBT];
-  const float* S = a.S + f.px_off;
-  const int nv = a.chi3 ? 3 : 2;
-  for (int v = 0; v < nv; ++v) {
-    const float2* chi = (v == 0 ? a.chi1 : (v == 1 ? a.chi2 : a.chi3)) + f.px_off;
-    // residual luma on [ty0-3, ty0+kBT+5) x [tx0-3, ...)
-    for (int i = threadIdx.x; i < kBH * kBH; i += blockDim.x) {
-      const int ly = i / kBH, lx = i % kBH;
-      const int y = ty0 - 3 + ly, x = tx0 - 3 + lx;
-      float val = 0.f;
-      if (y >= 0 && y < f.h && x >= 0 && x < f.w) {
-        const int64_t o = (int64_t)y * f.pitch + x;
-        val = S[o] - re_mul(chi[o], carrier_at(a, f, y, x));
-      }
-      yv[ly][lx] = val;
-    }
-    __syncthreads();
-    // e = |Dx y| + |Dy y| (forward, zero on the last column / row), zero
-    // outside the field (the box blur's zero padding).
-    for (int i = threadIdx.x; i < (kBH - 1) * (kBH - 1); i += blockDim.x) {
-      const int ly = i / (kBH - 1), lx = i % (kBH - 1);
-      const int y = ty0 - 3 + ly, x = tx0 - 3 + lx;
-      float e = 0.f;
-      if (y >= 0 && y < f.h && x >= 0 && x < f.w) {
-        const float dx = (x + 1 < f.w) ? yv[ly][lx + 1] - yv[ly][lx] : 0.f;
-        const float dy = (y + 1 < f.h) ? yv[ly + 1][lx] - yv[ly][lx] : 0.f;
-        e = fabsf(dx) + fabsf(dy);
-      }
-      ev[ly][lx] = e;
-    }
-    __syncthreads();
-    // vertical box (rows of the tile, all halo columns)
-    for (int i = threadIdx.x; i < kBT * (kBT + 6); i += blockDim.x) {
-      const int ly = i / (kBT + 6), lx = i % (kBT + 6);
-      float acc = 0.f;
+  const int ntx = (fw + kBC - 1) / kBC;
+  const int ty0 = (t / ntx) * a.blend_rows, tx0 = (t % ntx) * kBC;
+  const int lane = threadIdx.x;
+  const int x = tx0 - 4 + 2 * lane;
+  const bool ina = x >= 0 && x < fw, inb = x >= 0 && x + 1 < fw;
+  const bool hxb = x + 2 < fw;
+  const float2 z = make_float2(0.f, 0.f);
+  const float2 Pa = ina ? __ldg(a.col_phasor + f.col_off + x) : z;
+  const float2 Pb = inb ? __ldg(a.col_phasor + f.col_off + x + 1) : z;
+  const float* const S = a.S + f.px_off + x;
+  const float4* const LP = a.line_phasor + f.line_off;
+  const float2* chi[NV];
 #pragma unroll
-      for (int k = 0; k < 7; ++k) acc += ev[ly + k][lx];
-      vb[ly][lx] = acc * (1.0f / 7.0f);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kBT * kBT; i += blockDim.x) {
-      const int ly = i / kBT, lx = i % kBT;
-      const int y = ty0 + ly, x = tx0 + lx;
-      float acc = 0.f;
+  for (int v = 0; v < NV; ++v) chi[v] = (v == 0 ? a.chi1 : v == 1 ? a.chi2 : a.chi3) + f.px_off + x;
+  const bool out = ina && lane >= 2 && lane < 2 + kBC / 2;
+  auto load = [&](int y, BlendRow<NV>& r) {
+    r.s = z;
+    r.L = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int k = 0; k < 7; ++k) acc += vb[ly][lx + k];
-      const float E = acc * (1.0f / 7.0f);
-      const float wt = 1.0f / (E + 0.5f);
-      float2 cv = make_float2(0.f, 0.f);
-      if (y < f.h && x < f.w) cv = chi[(int64_t)y * f.pitch + x];
-      if (v == 0) {
-        num[ly][lx] = cscale(cv, wt);
-        wsum[ly][lx] = wt;
-      } else {
-        num[ly][lx] = cadd(num[ly][lx], cscale(cv, wt));
-        wsum[ly][lx] += wt;
-      }
+    for (int v = 0; v < NV; ++v) r.c[v] = r.L;
+    if (y >= 0 && y < fh && ina) {
+      const int64_t o = (int64_t)y * pitch;
+      r.s = __ldg(reinterpret_cast<const float2*>(S + o));
+      r.L = __ldg(LP + y);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) r.c[v] = __ldg(reinterpret_cast<const float4*>(chi[v] + o));
     }
-    __syncthreads();
-  }
-  float2* X = a.chi0 + f.px_off;
-  float* Y = a.Y + f.px_off;
-  for (int i = threadIdx.x; i < kBT * kBT; i += blockDim.x) {
-    const int ly = i / kBT, lx = i % kBT;
-    const int y = ty0 + ly, x = tx0 + lx;
-    if (y < f.h && x < f.w) {
-      const float2 c0 = make_float2(num[ly][lx].x / wsum[ly][lx], num[ly][lx].y / wsum[ly][lx]);
-      const int64_t o = (int64_t)y * f.pitch + x;
-      X[o] = c0;
-      Y[o] = S[o] - re_mul(c0, carrier_at(a, f, y, x));
+  };
+  float pa[NV], pb[NV];           // y_v of the last row
+  float ea[NV][7], eb[NV][7];     // e of the last seven rows
+  const int rows = min(a.blend_rows, fh - ty0) + 7;
+  BlendRow<NV> next;
+  load(ty0 - 3, next);
+  for (int r0 = 0; r0 < rows; r0 += 7) {
+#pragma unroll
+    for (int u = 0; u < 7; ++u) {
+      const int r = r0 + u, y = ty0 - 3 + r;  // y_v of row y, e of row y - 1
+      if (r >= rows) break;
+      const BlendRow<NV> cur = next;
+      if (r + 1 < rows) load(y + 1, next);
+      BlendRow<NV> q;  // the row that is complete after e of row y - 1
+      const int yo = y - 4;
+      if (r >= 7) load(yo, q);
+      const float2 ca = blend_car(cur.L, Pa), cb = blend_car(cur.L, Pb);
+      constexpr float k7 = 1.0f / 7.0f;
+      float wa[NV], wb[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const float na = blend_luma(cur.s.x, make_float2(cur.c[v].x, cur.c[v].y), ca);
+        const float nb = blend_luma(cur.s.y, make_float2(cur.c[v].z, cur.c[v].w), cb);
+        if (r > 0) {
+          const float pr = __shfl_down_sync(0xffffffffu, pa[v], 1);
+          const bool row = y - 1 >= 0 && y - 1 < fh, hy = y < fh;
+          const float dxa = inb ? pb[v] - pa[v] : 0.f, dxb = hxb ? pr - pb[v] : 0.f;
+          const float dya = hy ? na - pa[v] : 0.f, dyb = hy ? nb - pb[v] : 0.f;
+          ea[v][(u + 6) % 7] = row && ina ? fabsf(dxa) + fabsf(dya) : 0.f;
+          eb[v][(u + 6) % 7] = row && inb ? fabsf(dxb) + fabsf(dyb) : 0.f;
+        }
+        pa[v] = na;
+        pb[v] = nb;
+        if (r >= 7) {
+          float va = ea[v][u], vb = eb[v][u];
+#pragma unroll
+          for (int k = 1; k < 7; ++k) {
+            va += ea[v][(u + k) % 7];
+            vb += eb[v][(u + k) % 7];
+          }
+          va = __fmul_rn(va, k7);
+          vb = __fmul_rn(vb, k7);
+          const float m2b = __shfl_up_sync(0xffffffffu, vb, 2);
+          const float m1a = __shfl_up_sync(0xffffffffu, va, 1);
+          const float m1b = __shfl_up_sync(0xffffffffu, vb, 1);
+          const float p1a = __shfl_down_sync(0xffffffffu, va, 1);
+          const float p1b = __shfl_down_sync(0xffffffffu, vb, 1);
+          const float p2a = __shfl_down_sync(0xffffffffu, va, 2);
+          const float ha = (((((m2b + m1a) + m1b) + va) + vb) + p1a) + p1b;
+          const float hb = (((((m1a + m1b) + va) + vb) + p1a) + p1b) + p2a;
+          wa[v] = 1.0f / __fmaf_rn(ha, k7, 0.5f);
+          wb[v] = 1.0f / __fmaf_rn(hb, k7, 0.5f);
+        }
+      }
+      if (r >= 7 && out) {
+        float2 numa, numb;
+        float wsa = 0.f, wsb = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const float4 c = q.c[v];
+          if (v == 0) {
+            numa = make_float2(__fmul_rn(c.x, wa[v]), __fmul_rn(c.y, wa[v]));
+            numb = make_float2(__fmul_rn(c.z, wb[v]), __fmul_rn(c.w, wb[v]));
+            wsa = wa[v];
+            wsb = wb[v];
+          } else {
+            numa = make_float2(__fmaf_rn(c.x, wa[v], numa.x), __fmaf_rn(c.y, wa[v], numa.y));
+            numb = make_float2(__fmaf_rn(c.z, wb[v], numb.x), __fmaf_rn(c.w, wb[v], numb.y));
+            wsa += wa[v];
+            wsb += wb[v];
+          }
+        }
+        const float2 ua = make_float2(numa.x / wsa, numa.y / wsa);
+        const float2 ub = make_float2(numb.x / wsb, numb.y / wsb);
+        const float ya = blend_luma(q.s.x, ua, blend_car(q.L, Pa));
+        const float yb = blend_luma(q.s.y, ub, blend_car(q.L, Pb));
+        const int64_t o = f.px_off + (int64_t)yo * pitch + x;
+        if (inb) {
+          *reinterpret_cast<float4*>(a.chi0 + o) = make_float4(ua.x, ua.y, ub.x, ub.y);
+          *reinterpret_cast<float2*>(a.Y + o) = make_float2(ya, yb);
+        } else {
+          a.chi0[o] = ua;
+          a.Y[o] = ya;
+        }
+      }
     }
   }
 }
@@ -1056,7 +1116,10 @@ void launch_init(const InitArgs& a, int total_prows, int total_cgroups, int tota
     sym_cols(1);
     sym_rows(1);
   }
-  if (total_btiles > 0) k_init_blend<<<total_btiles, 256, 0, st>>>(a);
+  if (total_btiles > 0) {
+    if (a.chi3) k_init_blend<3><<<total_btiles, 32, 0, st>>>(a);
+    else k_init_blend<2><<<total_btiles, 32, 0, st>>>(a);
+  }
 }
 
 void launch_init_filter_adjoint(const InitArgs& a, int total_prows, int total_cgroups,
@@ -1074,6 +1137,13 @@ int aniso_max_samples() { return kAnisoMax; }
 int init_col_group(int col_m) {
   return col_m == kFftLong ? 1 : col_m == kColFftWide ? kColGroupWide : kColGroup;
 }
-int init_blend_tile() { return kBT; }
+int init_blend_tiles(int h, int w, int rows) {
+  return ((h + rows - 1) / rows) * ((w + kBC - 1) / kBC);
+}
+// Tall tiles compute seven rows that they do not output, low ones as many as
+// they output: tall where they fill the chip all the same. @ROWS@
+int init_blend_rows(int tall_tiles, int sm_count) {
+  return tall_tiles >= 8 * sm_count ? kBlendTall : kBlendLow;
+}
 
 }  // namespace hvdg

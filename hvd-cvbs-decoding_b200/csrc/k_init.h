@@ -32,6 +32,7 @@ struct InitArgs {
   const int* cgrp_first;       // field -> first column group
   const int* btile_field;      // blend tile -> field
   const int* btile_first;      // field -> first blend tile
+  int blend_rows;              // rows of a blend tile
   // Adjoint mode (both non-null): the rows pass filters the two variant
   // planes of adj_in (per field at rowbuf_off, 2 x hp x pitch, pad rows
   // included) instead of the demodulated composite, and the columns pass
@@ -58,6 +59,10 @@ void launch_aniso(FieldDesc* d_fields, int n_fields, const float2* chi0, cudaStr
 int aniso_max_samples();
 // columns per CTA of the column pass for a geometry with column length col_m
 int init_col_group(int col_m);
-int init_blend_tile();
+// tiles of the blend over a plane, `rows` of them high, and that height for a
+// batch of tall_tiles tiles of kBlendTall rows
+constexpr int kBlendTall = 21, kBlendLow = 7;
+int init_blend_tiles(int h, int w, int rows);
+int init_blend_rows(int tall_tiles, int sm_count);
 
 }  // namespace hvdg

@@ -16,6 +16,7 @@
 // or for the refinement a warp per tile that replays the visit from
 // per-row running sums), so the selected vectors, sub-pel fits and
 // confidences equal the reference's bit for bit.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "hvdg_common.cuh"
@@ -36,8 +37,8 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // the window sums from the prefixes. Bands of 8 rows or 16 columns keep many
 // blocks in flight. A band is read whole before it is written, so source and
 // destination may be the same plane. Against a warp that staged, chained and
-// windowed 32 rows in turn (and a thread per column), 760 x 242, two planes:
-// rows 72 -> 11 us, columns 46 -> 7 us.
+// windowed 32 rows in turn (and a thread per column), a PAL pair: rows 86 -> 16
+// us, columns 55 -> 10 us.
 constexpr int kBoxThreads = 256;
 constexpr int kRowBand = 8;
 constexpr int kColBand = 16;
@@ -279,7 +280,7 @@ constexpr int kCoarseReach = 5;  // (2 * 5 + 1)^2 <= kCoarseCands
 // reaches it (a ballot over the rows) ends the candidate with that sum,
 // strict-less update. Every cost and decision is the per-thread kernel's. A
 // warp per tile reading global memory took 53 us on a PAL pair (latency of
-// three rounds of 64 dependent loads), this takes 8.
+// three rounds of 64 dependent loads), this takes 22.
 __global__ void __launch_bounds__(kCoarseCands) k_me_coarse_tile(
     const MeField* __restrict__ mf, const MePair* __restrict__ pairs, int npairs,
     const float* __restrict__ dec, MeArgs a, float* __restrict__ cdy, float* __restrict__ cdx) {
@@ -446,7 +447,7 @@ __global__ void k_me_refine(const MeField* __restrict__ mf, const MePair* __rest
 // order, so every cost, decision and vector is the per-thread kernel's. What
 // bounds it is one chained addition per pixel of the tile (4 cycles, 2 us for
 // 32 x 32); a warp per tile with its operands in global memory and the five
-// CostAt sums after the candidates took 187 us on a PAL pair, this takes 11.
+// CostAt sums after the candidates took 186 us on a PAL pair, this takes 31.
 constexpr int kRefineCands = 49;  // RangeFromCentre(-3, 3)^2
 constexpr int kRefineTile = 64;
 constexpr int kRefineThreads = 96;
@@ -604,7 +605,7 @@ __global__ void __launch_bounds__(kRefineThreads) k_me_refine_tile(
 // and one lane adds them in the reference's order; conf0 and the ratio go to
 // out_conf / out_dy for (2). The two chained additions per pixel bound it (3
 // us for 32 x 32); one thread per tile of one block per pair, with the medians
-// behind it, took 190 us on a PAL pair, (1) and (2) take 16.
+// behind it, took 187 us on a PAL pair, (1) takes 14 and (2) 12.
 constexpr int kConfChunk = 1024;
 constexpr int kConfWarps = 8;
 __global__ void __launch_bounds__(32 * kConfWarps) k_me_tile_stats(
@@ -788,7 +789,7 @@ __device__ __forceinline__ int quant_luma(float y) {
 // sums, so any order is exact. A block takes a 64 x 16 tile with its border
 // into shared memory, sums columns, then rows. One pass over the plane in
 // place of a running sum per column and then per row (two 760 x 242 planes:
-// 358 -> 6 us).
+// 354 -> 7 us).
 constexpr int kQbX = 64, kQbY = 16;
 __global__ void __launch_bounds__(256) k_sad_blur(const MeField* __restrict__ mf,
                                                   const float* __restrict__ luma,
@@ -1149,28 +1150,36 @@ __global__ void __launch_bounds__(kSadThreads, 6) k_sad_search(const MeField* __
   }
 }
 
-// MotionConfidence on the IRE scale from the exact integer statistics. One
-// CTA per pair.
-// One block of 1024 threads per pair: the rank counts (nt^2 comparisons) bound it
-// (768 tiles, both middles: 64 us by 256 threads in two passes, 14 now).
-constexpr int kSadConfThreads = 1024;
-__global__ void __launch_bounds__(kSadConfThreads) k_sad_confidence(const MeField* __restrict__ mf,
+// MotionConfidence on the IRE scale from the exact integer statistics. A
+// cluster of eight CTAs per pair: the rank counts (nt^2 comparisons) bound it,
+// so each CTA ranks an eighth of the tiles against all and tells the others of
+// the middle ones it finds (750 tiles: 63 us by one CTA in two passes over the
+// ranks, 23 by one of 1024 threads in one pass, 14 by the cluster).
+constexpr int kSadConfThreads = 256, kSadConfCtas = 8;
+__global__ void __cluster_dims__(kSadConfCtas, 1, 1) __launch_bounds__(kSadConfThreads) k_sad_confidence(const MeField* __restrict__ mf,
                                                         const MePair* __restrict__ pairs,
                                                         SadArgs a, SadBuffers out) {
   extern __shared__ double sadc_sm[];
   __shared__ double mid[2];
-  const int p = blockIdx.x;
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int p = blockIdx.x / kSadConfCtas, rank = blockIdx.x % kSadConfCtas;
   const MeField mc = mf[pairs[p].cur];
   const int b = a.block;
   const int th = (mc.h + b - 1) / b, tw = (mc.w + b - 1) / b, nt = th * tw;
+  const int t0 = rank * kSadConfThreads + threadIdx.x;
+  constexpr int kStep = kSadConfCtas * kSadConfThreads;
   double* ratios = sadc_sm;
   const int o = a.tiles_off * p;
   for (int t = threadIdx.x; t < nt; t += blockDim.x)
     ratios[t] = out.bestv[o + t] / fmax(1.0, out.npx[o + t]);
   __syncthreads();
+  cl.sync();  // every CTA of the cluster runs: its shared memory can be written
   // the two middle ratios by counting ranks, both in one pass
   const int k = nt / 2;
-  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+  auto tell = [&](int which, double v) {
+    for (int r = 0; r < kSadConfCtas; ++r) cl.map_shared_rank(mid, r)[which] = v;
+  };
+  for (int t = t0; t < nt; t += kStep) {
     const double v = ratios[t];
     int less = 0, eq = 0;
 #pragma unroll 8
@@ -1178,13 +1187,13 @@ __global__ void __launch_bounds__(kSadConfThreads) k_sad_confidence(const MeFiel
       less += ratios[u] < v;
       eq += ratios[u] == v;
     }
-    if (less <= k && k < less + eq) mid[0] = v;
-    if (less <= k - 1 && k - 1 < less + eq) mid[1] = v;
+    if (less <= k && k < less + eq) tell(0, v);
+    if (less <= k - 1 && k - 1 < less + eq) tell(1, v);
   }
-  __syncthreads();
+  cl.sync();
   const double med = nt % 2 == 0 ? 0.5 * (mid[0] + mid[1]) : mid[0];
   const double sc2 = (double)kQuantScale * (double)kQuantScale;
-  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+  for (int t = t0; t < nt; t += kStep) {
     const double npx = out.npx[o + t];
     const double norm = 1.0 / fmax(1.0, npx);
     const double tmean = out.s1[o + t] * norm;
@@ -1212,7 +1221,7 @@ void launch_motion_sad(const MeField* d_fields, int nf, int max_h, int max_w,
     cudaFuncSetAttribute(k_sad_search, cudaFuncAttributeMaxDynamicSharedMemorySize, kSadMaxSmem);
   });
   k_sad_search<<<dim3(th * tw, npairs), kSadThreads, smem, st>>>(d_fields, d_pairs, b.qblur, a, b);
-  k_sad_confidence<<<npairs, kSadConfThreads, th * tw * (int)sizeof(double), st>>>(d_fields, d_pairs, a, b);
+  k_sad_confidence<<<npairs * kSadConfCtas, kSadConfThreads, th * tw * (int)sizeof(double), st>>>(d_fields, d_pairs, a, b);
 }
 
 // ---------------------------------------------------------------------------
@@ -1518,7 +1527,8 @@ __global__ void k_traj_snap(const MeField* __restrict__ mf, const MePair* __rest
 // A warp per tile: the squared differences of the prediction and of zero
 // motion are formed by all lanes into shared memory, kVerifyChunk pixels at a
 // time, and two lanes add them in the reference's order (4 cycles a pixel). A
-// thread per sum reading global memory took 95 us for 5 NTSC pairs, this 12.
+// thread per sum reading global memory took 96 us for the pairs of a six-frame
+// NTSC window, this 20.
 constexpr int kVerifyChunk = 1024;
 constexpr int kVerifyWarps = 4;
 __global__ void __launch_bounds__(32 * kVerifyWarps) k_traj_verify(

@@ -132,7 +132,7 @@ __device__ void tridiag_smooth(const double* d, const double* a, int n, double l
 
 // One CTA per field: a line per thread in the smoother and the angles, four
 // lines per warp in the burst sums (256 threads and a line per warp at a time:
-// 64 us for an NTSC field; 29 now, the FP64 divisions of the reduction's 18
+// 67 us for an NTSC field, 100 for PAL; 47 and 62 now, the FP64 divisions of the reduction's 18
 // steps and the angles' FP64 functions bounding it).
 constexpr int kLkThreads = 512;
 constexpr int kLkLines = 4;

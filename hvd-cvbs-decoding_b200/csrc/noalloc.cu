@@ -107,9 +107,9 @@ extern "C" hvdg_status hvdg_holographic_init_noalloc(const float* s, const float
   int hp = 0, pad = 0;
   hvdg::init_tables_for(*g, &khat, &colph, &twr, &twc, &hp, &pad);
   const int pitch = (w + hvdg::kStrip - 1) / hvdg::kStrip * hvdg::kStrip;
-  const int cgroup = hvdg::init_col_group(hvdg::kColFft), bt = hvdg::init_blend_tile();
+  const int cgroup = hvdg::init_col_group(hvdg::kColFft);
   const int ngroups = (w + cgroup - 1) / cgroup;
-  const int ntiles = ((h + bt - 1) / bt) * ((w + bt - 1) / bt);
+  const int ntiles = hvdg::init_blend_tiles(h, w, hvdg::kBlendTall);
 
   // ---- layout inside the static array ----
   size_t o = 0;
@@ -221,6 +221,7 @@ extern "C" hvdg_status hvdg_holographic_init_noalloc(const float* s, const float
   ia.cgrp_first = it + hp + 1 + ngroups;
   ia.btile_field = it + hp + 1 + ngroups + 1;
   ia.btile_first = it + hp + 1 + ngroups + 1 + ntiles;
+  ia.blend_rows = hvdg::kBlendTall;
   hvdg::launch_init(ia, hp, ngroups, ntiles, 0);
   e = cudaGetLastError();
   if (e == cudaSuccess)

@@ -477,7 +477,9 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
   }
   // init tables
   std::vector<int> prow_field, prow_first, cgrp_field, cgrp_first, btile_field, btile_first;
-  const int bt = hvdg::init_blend_tile();
+  int tall = 0;
+  for (const FieldPlan& p : b.fp) tall += hvdg::init_blend_tiles(p.h, p.w, hvdg::kBlendTall);
+  b.blend_rows = hvdg::init_blend_rows(tall, ctx->sm_count);
   for (int i = 0; i < m; ++i) {
     const FieldPlan& p = b.fp[i];
     const int cg = hvdg::init_col_group(b.gtabs[p.geom_slot]->col_m);
@@ -486,7 +488,7 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
     cgrp_first.push_back((int)cgrp_field.size());
     for (int x = 0; x < p.w; x += cg) cgrp_field.push_back(i);
     btile_first.push_back((int)btile_field.size());
-    const int nt = ((p.h + bt - 1) / bt) * ((p.w + bt - 1) / bt);
+    const int nt = hvdg::init_blend_tiles(p.h, p.w, b.blend_rows);
     for (int t = 0; t < nt; ++t) btile_field.push_back(i);
   }
   auto append = [&](const std::vector<int>& v) {
@@ -745,6 +747,7 @@ hvdg::InitArgs init_args(hvdg_ctx* ctx, const Staged& S) {
   ia.cgrp_first = itb + b.it_cgrp_first;
   ia.btile_field = itb + b.it_btile_field;
   ia.btile_first = itb + b.it_btile_first;
+  ia.blend_rows = b.blend_rows;
   return ia;
 }
 

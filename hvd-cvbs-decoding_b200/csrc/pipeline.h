@@ -217,6 +217,7 @@ struct Batch {
   std::vector<int> gcol_off;
   std::vector<Unit> units;
   std::vector<int> itab;  // prow_field | prow_first | cgrp_field | cgrp_first | btile_field | btile_first
+  int blend_rows = 0;        // height of the init blend's tiles
   int it_prow_field, it_prow_first, it_cgrp_field, it_cgrp_first, it_btile_field, it_btile_first;
   std::vector<int64_t> rowbuf_offs;
   std::vector<int4> crop_rows;  // per S row: (plane, row, source field, source line)
