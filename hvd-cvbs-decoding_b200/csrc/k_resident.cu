@@ -456,7 +456,7 @@ __device__ __forceinline__ void warp_sum6(const double v[kNV], int lane, double&
 }
 
 // n / d to within a rounding or two of FP64, for the scalar step's critical
-// path (the FP64 division measured 408 cycles there, this ~150): Newton's
+// path (the FP64 division measured 408 cycles there): Newton's
 // iteration for the reciprocal from a single-precision seed, then one residual
 // correction of the quotient. Outside the seed's range, the division itself.
 __device__ __forceinline__ double quotient(double n, double d) {

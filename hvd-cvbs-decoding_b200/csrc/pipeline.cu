@@ -256,9 +256,9 @@ std::vector<hvdg::SolveShape> solve_shapes(const hvdg_field_in* in, int n, const
   return v;
 }
 
-// The resident launches of a set of planes, one per plane size (a launch's
-// tiles all have its tallest tile's register rows, so sizes are not mixed: a
-// batch of 40 NTSC and 24 PAL fields takes 55 ms in two launches, 64 in one).
+// The resident launches of a set of planes, one per plane size: the gangs of a
+// launch are as many as its largest plane allows, so sizes are not mixed (NTSC
+// fields run four at a time, PAL fields three).
 // Empty when one of them does not fit the chip.
 std::vector<ResidentGroup> resident_groups(hvdg_ctx* ctx,
                                            const std::vector<hvdg::SolveShape>& shapes, bool nbr,
