@@ -13,9 +13,10 @@ temporal terms off. Synthetic data (hvdg.synth), seeded per rank.
               pinned uint16 inputs in, float Y/chi out, copies included,
               wall clock of the synchronous call.
   plain     : the one-field-per-launch path (hvdg_set_batching(ctx, 0)).
-  roofline  : the IRLS+CG solver kernel, algorithmic bytes (92 B per active
-              px per CG iteration + 80 B per active px per IRLS outer) over
-              its event-timed duration, against the measured HBM copy peak.
+  roofline  : the IRLS+CG solver, arithmetic (84 operations per active px
+              per CG iteration + 120 per active px per IRLS outer) over its
+              event-timed duration, against the FP32 pipes' rate at the SM
+              clock seen: its state stays on chip, so HBM does not bound it.
   cpu_baseline : the reference engine (oracle/_ref, compiled from the
               reference sources) on a bounded sample of the same workload on
               the host cores (one quarter of the fields, counted by solver
@@ -49,8 +50,11 @@ sys.path.insert(0, str(REPO))
 
 METRIC = "fields/s on 1 B200, batched FP32 vs plain per-field GPU, at <=0.05 dB PSNR delta"
 N_NTSC, N_PAL = 40, 24
-ALG_BYTES_ITER = 92.0    # per active px per CG iteration
-ALG_BYTES_OUTER = 80.0   # per active px per IRLS outer
+# operations per active px of a CG iteration: direction, residual and chi updates
+# 12, carrier 8, luma part 4, differences 6, fluxes 6, divergence 18, curvature
+# 14, four inner products 16; and of an IRLS outer (weights, gradient)
+ALG_OPS_ITER, ALG_OPS_OUTER = 84.0, 120.0
+FP32_OPS_PER_SM_CLOCK = 256.0  # 128 lanes, a fused multiply-add counting two
 
 
 WORKLOADS = {
@@ -103,22 +107,14 @@ def solver_config():
     return api.default_config(fast=0, cg_tol=1e-6, temporal_strength=-1.0)
 
 
-def measured_peaks():
-    p = REPO / "MEASURED_PEAKS.json"
-    if p.exists():
-        d = json.loads(p.read_text())
-        return float(d["hbm_gbs"]), "measured"
-    return 6650.0, "fallback"
-
-
 def profile_traffic(name):
-    """Per-launch DRAM traffic of the solver on the mixed-64 workload, from
+    """DRAM traffic of the solver on one mixed-64 batch, from
     the committed ncu summary (profiles/solver_traffic.json); None for the
     other workloads (not captured) or without the summary."""
     p = REPO / "profiles" / "solver_traffic.json"
     if name == "mixed64" and p.exists():
         try:
-            return json.loads(p.read_text()).get("bytes_per_launch")
+            return json.loads(p.read_text()).get("bytes_per_batch")
         except Exception:
             return None
     return None
@@ -140,7 +136,7 @@ class ClockSampler:
             self.fh = open(self.path, "w")
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.index}", f"--query-gpu={self.Q}", "--format=csv,noheader,nounits",
-                 "-lms", "200"], stdout=self.fh, stderr=subprocess.DEVNULL)
+                 "-lms", "50"], stdout=self.fh, stderr=subprocess.DEVNULL)
         except Exception:
             self.proc = None
 
@@ -756,17 +752,19 @@ def main():
                  "ms_per_step": pt / psteps}
 
     value = throughput(n, args.steps, world, ms_total)
-    peak, peak_kind = measured_peaks()
-    alg_bytes_per_launch = (ALG_BYTES_ITER * pix_iters + ALG_BYTES_OUTER * pix_outers) / args.steps
+    alg_ops = (ALG_OPS_ITER * pix_iters + ALG_OPS_OUTER * pix_outers) / args.steps
     solver_s = ms_solver / 1000.0 / args.steps
-    achieved = alg_bytes_per_launch / solver_s / 1e9
-    roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    achieved = alg_ops / solver_s / 1e12
+    sm_mhz = (clocks or {}).get("sm_mhz") or 1965.0
+    peak = (torch.cuda.get_device_properties(0).multi_processor_count * FP32_OPS_PER_SM_CLOCK *
+            sm_mhz * 1e6 / 1e12)
+    roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "traffic": profile_traffic(args.workload),
             "traffic_source": "committed one-pass ncu capture of this solver build on this workload "
                               "(profiles/solver_traffic.json), not measured in this run",
-            "peak_kind": peak_kind,
-            "kernel": "k_solver (persistent IRLS + CG)",
-            "alg_bytes_per_launch": alg_bytes_per_launch, "ms_per_launch": 1000 * solver_s}
+            "peak_kind": "FP32 lanes at the SM clock seen",
+            "kernel": "k_resident (IRLS + CG, a field's state on chip)",
+            "alg_ops_per_batch": alg_ops, "ms_per_batch": 1000 * solver_s}
 
     line = {
         "metric": METRIC, "value": value, "unit": "fields/s", "n_gpus": world,

@@ -459,7 +459,7 @@ hvdg_status decode_adjoint_chunk(hvdg_ctx* ctx, const hvdg_field_in* fields, int
     for (int i = 0; i < 4; ++i) scalar_bar[i] += accv[4 * j + i];
   if (diag) {
     diag->cg_iterations_run += cg_run + adj_run;
-    diag->kernel_launches += 8 + n_outer * 7 + 12;
+    diag->kernel_launches += 18 + n_outer * (5 + 2 * std::max<int>(1, S.b.rg.size()));
   }
   return HVDG_OK;
 }

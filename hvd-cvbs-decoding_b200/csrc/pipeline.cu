@@ -973,7 +973,7 @@ hvdg_status run_batch_once(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const 
     const cudaError_t e =
         launch_solve(ctx, S, sa, S.b.rg, false, opt.ctas_per_sm);
     if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
-    S.launches += 1;
+    S.launches += std::max<int>(1, S.b.rg.size());
   }
   mark(ctx, 3);
   const cudaError_t le = cudaGetLastError();
@@ -1086,6 +1086,7 @@ hvdg_status run_batch_graph(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const
     ctx->gsig = sig;
     ctx->gepoch = ctx->epoch;
     ctx->gn = n;
+    ctx->g_solves = std::max<int>(1, S.b.rg.size());
     ctx->g_pix.assign(n, 0);
     ctx->g_outer.assign(n, 0);
     for (int i = 0; i < n; ++i) {
@@ -1118,7 +1119,7 @@ hvdg_status graph_result(hvdg_ctx* ctx, hvdg_diag* diag) {
       diag->solver_pixel_iters += (int64_t)ctl[i].cg_iters * ctx->g_pix[i];
       diag->solver_pixel_outers += (int64_t)ctx->g_outer[i] * ctx->g_pix[i];
     }
-    diag->kernel_launches += 7;
+    diag->kernel_launches += 6 + ctx->g_solves;
   }
   if (ctx->flags_host[1]) {
     ctx->last_error = "non-finite input samples";

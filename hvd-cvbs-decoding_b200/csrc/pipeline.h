@@ -135,6 +135,7 @@ struct hvdg_ctx {
   void* ctl_host = nullptr;      // pinned FieldCtl[ctl_host_n]
   int ctl_host_n = 0;
   int gn = 0;                    // fields of the cached graph
+  int g_solves = 1;              // its solver launches
   std::vector<int64_t> g_pix;    // per-field active px of the cached graph
   std::vector<int> g_outer;      // per-field IRLS outers of the cached graph
   // autotuner: batch signature -> (band rows, CTAs per SM)

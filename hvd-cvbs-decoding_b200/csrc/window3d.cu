@@ -511,11 +511,13 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
           // the consensus snap, which is re-applied: same inputs, same result)
           hvdg::launch_motion_cache(d_gid, npairs, nt, nt, mb.dy, mb.dx, mb.conf, mcache, mc_stride,
                                     false, s);
+          S.launches += 1;
         } else {
           if (sad_me)
             hvdg::launch_motion_sad(d_mf, nf, h, w, d_mp, n_full, sad_a, sad_b, s);
           else
             hvdg::launch_motion(d_mf, nf, h, w, d_mp, n_full, ma, mb, s);
+          S.launches += sad_me ? 3 : 7;
           const int npred = npairs - n_full;
           if (npred > 0) {
             const int64_t ofs = (int64_t)n_full * nt;
@@ -525,11 +527,13 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
             hvdg::launch_me_confidence(d_mf, d_mp + n_full, npred, h, w, ma, mb.blur, mb.mdy + ofs,
                                        mb.mdx + ofs, mb.sdy + ofs, mb.sdx + ofs, mb.best + ofs,
                                        mb.dy + ofs, mb.dx + ofs, mb.conf + ofs, s);
-            S.launches += 2;
+            S.launches += 3;
           }
-          if (cfg.fast && n_passes > 1)
+          if (cfg.fast && n_passes > 1) {
             hvdg::launch_motion_cache(d_gid, npairs, nt, nt, mb.dy, mb.dx, mb.conf, mcache,
                                       mc_stride, true, s);
+            S.launches += 1;
+          }
         }
         if (joint_pass) {
           // the anchor blends with the pairwise motion as estimated (before
@@ -550,7 +554,7 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
           S.launches += 1;
         }
         hvdg::launch_vectors(d_mf, d_mp, npairs, h, w, ma, vb, cfg.fast != 0, s);
-        S.launches += 8;
+        S.launches += cfg.fast ? 5 : 3;
         if (gate_cfg && !(cfg.fast && pass == 0)) {
           // coherence gate against the current chi of both fields
           hvdg::CohBuffers cb;
@@ -562,7 +566,7 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
           cb.pix_off = d_pix_off;
           cb.chan_stride = coh_stride;
           hvdg::launch_coherence_gate(d_mf, d_mp, npairs, h, w, ma, cb, cfg.coherence_gate, s);
-          S.launches += 10;
+          S.launches += 4;
         }
         if (!env_list.empty()) {
           e = cudaMemcpyAsync(d_list, env_list.data(), sizeof(int) * env_list.size(),
@@ -574,7 +578,7 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
           hvdg::launch_envelope(at<FieldDesc>(ctx, L.o_fields), d_list, (int)env_list.size(), h, w,
                                 at<float>(ctx, L.o_Y), at<float2>(ctx, L.o_X0), eb, e2, floor_max,
                                 s);
-          S.launches += 5;
+          S.launches += 4;
         }
         hvdg::launch_nbr_assemble(at<FieldDesc>(ctx, L.o_fields), d_np, npairs, h, w,
                                   at<float>(ctx, L.o_S), at<float4>(ctx, L.o_lineph),
@@ -722,7 +726,7 @@ hvdg_status decode_window_3d(hvdg_ctx* ctx, const hvdg_field_in* in, int nf,
         sa.n_phases = cphases[ci];
         e = launch_solve(ctx, S, sa, crg[ci], has_temporal);
         if (e != cudaSuccess) return hvdg::cuda_fail(ctx, e, "solver launch");
-        S.launches += 2;
+        S.launches += 1 + std::max<int>(1, crg[ci].size());
       }
       // the solved fields' luma / chi now replace their init state (Ys[j], chis[j])
     }

@@ -230,9 +230,13 @@ const char* hvdg_last_error(const hvdg_ctx* ctx);
 /* 0 = plain path (one field per launch sequence), 1 = batched persistent
  * launch (default). Exists for the batched-vs-plain comparison. */
 hvdg_status hvdg_set_batching(hvdg_ctx* ctx, int batched);
-/* Solver tiling: band height (rows per work unit; 0 = autotuned). */
+/* Tiling of the streaming solver: band height (rows per work unit) and CTAs per
+ * SM. 0, 0 (the default) leaves the choice to the library: planes whose state
+ * fits on the chip go to the resident solver, the others to the streaming one
+ * at autotuned bands. Any other value selects the streaming solver. */
 hvdg_status hvdg_set_tuning(hvdg_ctx* ctx, int band_rows, int ctas_per_sm);
-/* Bound of the solver's device-side waits on a field's phase flag, in polls
+/* Bound of the solvers' device-side waits (on a field's phase flag, or on another
+ * CTA's part of an exchange), in polls
  * (~0.5 us each; <= 0 restores the default 4,000,000, ~2 s). A wait that
  * runs out ends the launch and the call returns HVDG_ERR_DEVICE_TIMEOUT; the
  * context stays usable. No reference counterpart (the reference's CPU loops
