@@ -232,25 +232,30 @@ struct Tile {
   float2 Pa, Pb;        // column phasors
 };
 
+// A predicated store, so that the lanes of a warp stay together (branches around
+// the stores, and __syncwarp after them in every row, cost 0.1 to 0.3 us a sweep).
+__device__ __forceinline__ void st_slot_if(bool p, Slot* out, float2 v, unsigned long long tag) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 d;\n .reg .b128 t;\n setp.ne.s32 p, %4, 0;\n"
+      " mov.b64 d, {%1, %2};\n mov.b128 t, {d, %3};\n"
+      " @p st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(out),
+      "f"(v.x), "f"(v.y), "l"(tag), "r"((int)p)
+      : "memory");
+}
+
 // Publish row i (of nrow) of a warp: the tile's first and last rows go whole
 // to the neighbours above and below, lane 0 and lane 31 carry the side columns.
 __device__ __forceinline__ void publish_row(const Tile& t, Slot* out, int lane, int i,
                                             unsigned long long tag, float2 a, float2 b) {
   if (i == 0 && t.pub_up) {
-    if (t.va) st_slot(out + 2 * lane, pack2(a), tag);
-    if (t.vb) st_slot(out + 2 * lane + 1, pack2(b), tag);
+    st_slot_if(t.va, out + 2 * lane, a, tag);
+    st_slot_if(t.vb, out + 2 * lane + 1, b, tag);
   }
   if (i == t.pub_down) {
-    if (t.va) st_slot(out + kStrip + 2 * lane, pack2(a), tag);
-    if (t.vb) st_slot(out + kStrip + 2 * lane + 1, pack2(b), tag);
+    st_slot_if(t.va, out + kStrip + 2 * lane, a, tag);
+    st_slot_if(t.vb, out + kStrip + 2 * lane + 1, b, tag);
   }
-  const float2 e = lane == 0 ? a : b;
-  asm volatile(
-      "{\n .reg .pred p;\n .reg .b64 d;\n .reg .b128 t;\n setp.ge.s32 p, %4, 0;\n"
-      " mov.b64 d, {%1, %2};\n mov.b128 t, {d, %3};\n"
-      " @p st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(out + t.side + i),
-      "f"(e.x), "f"(e.y), "l"(tag), "r"(t.side)
-      : "memory");
+  st_slot_if(t.side >= 0, out + t.side + i, lane == 0 ? a : b, tag);
 }
 
 __device__ __forceinline__ bool poll_slot(const Slot* p, unsigned long long tag,
@@ -266,10 +271,11 @@ __device__ __forceinline__ bool poll_slot(const Slot* p, unsigned long long tag,
 
 // Tensor memory as a second register file: what a thread alone reads and writes
 // -- g, q and chi of its two pixels in each row, four words each -- moved by
-// one instruction per row and waited for where it is used. With g and q in
+// one instruction per row (the whole warp at once: __syncwarp before it where
+// lanes may have parted) and waited for where it is used. With g and q in
 // registers (56 of 128 at seven rows) and chi in shared memory the sweep
-// spilled, and took 5.4 us at 61 rows, 7.5 at 81 and 8.6 at 97; this takes 4.8,
-// 5.6 and 6.2, and the shared memory freed holds 112 rows instead of 97.
+// spilled, and took 5.4 us at 61 rows, 7.5 at 81 and 8.6 at 97; this takes 4.6,
+// 5.4 and 6.0, and the shared memory freed holds 112 rows instead of 97.
 constexpr uint32_t kTg = 0, kTq = 4, kTc = 8, kTRow = 12;
 __device__ __forceinline__ void tmem_st4(uint32_t a, float2 u, float2 v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a),
@@ -672,6 +678,7 @@ __global__ void __launch_bounds__(kRT, 1)
     }
     const Rows rw(M, t.rb, lane);
     constexpr uint32_t WB = Smem<kNbr>::kWB;
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
       if (i >= t.nrow) break;
@@ -698,6 +705,7 @@ __global__ void __launch_bounds__(kRT, 1)
       {
         Slot* out = reinterpret_cast<Slot*>(xb + my_edges + set * kSetBytes);
         const unsigned long long tag = tag_hi | ex;
+        __syncwarp();
 #pragma unroll 1
         for (int i = 0; i < t.nrow; ++i) {
           float2 xa, xb2;
@@ -719,6 +727,7 @@ __global__ void __launch_bounds__(kRT, 1)
           sts2(rw.yl + i * kUB, make_float2(ya, yb));
           publish_row(t, out, lane, i, tag, xa, xb2);
         }
+        tmem_wait_st();
         if (hrole) {
           unsigned long long lo;
           if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo, A.phase_wait_limit)) M.word[0] = 1;
@@ -728,7 +737,6 @@ __global__ void __launch_bounds__(kRT, 1)
         }
       }
       pending = 0;
-      tmem_wait_st();
       __syncthreads();
       // ---- weights (lagged diffusivity), neighbour data term ----
       ++ex;
@@ -852,6 +860,7 @@ __global__ void __launch_bounds__(kRT, 1)
         Slot* out = reinterpret_cast<Slot*>(xb + my_edges + set * kSetBytes);
         const unsigned long long tag = tag_hi | ex;
         Carry c;
+        __syncwarp();
         if (t.nrow > 0) carry_init(M, rw, t.rb, lane, c);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
@@ -882,13 +891,13 @@ __global__ void __launch_bounds__(kRT, 1)
           pgg0 += (double)cnorm(oa) + (double)cnorm(ob);
           publish_row(t, out, lane, i, tag, oa, ob);
         }
+        tmem_wait_st();
         if (hrole) {
           unsigned long long lo;
           if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo, A.phase_wait_limit)) M.word[0] = 1;
           hg = unpack2(lo);
           hd = make_float2(-hg.x, -hg.y);
         }
-        tmem_wait_st();
       }
       __syncthreads();
       bad = M.word[0] != 0;
@@ -898,6 +907,7 @@ __global__ void __launch_bounds__(kRT, 1)
       for (int k = 0; k < n_inner; ++k) {
         const bool first = k == 0;
         // the pending step and the new direction, own pixels then halo
+        __syncwarp();
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
           if (i >= t.nrow) break;
@@ -931,11 +941,11 @@ __global__ void __launch_bounds__(kRT, 1)
           sts2(rw.yl + i * kUB,
                make_float2(-re_rn(ua, car_rn(L, t.Pa)), -re_rn(ub, car_rn(L, t.Pb))));
         }
+        tmem_wait_st();
         if (hrole) {
           sts2(hu, hd);
           sts1(hyp, -re_rn(hd, hc));
         }
-        tmem_wait_st();
         __syncthreads();
         // ---- q = A d, the curvature and the inner products ----
         ++ex;
@@ -946,6 +956,7 @@ __global__ void __launch_bounds__(kRT, 1)
         pgg0 = 0.0;
         {
           Carry c;
+          __syncwarp();
           if (t.nrow > 0) carry_init(M, rw, t.rb, lane, c);
 #pragma unroll
           for (int i = 0; i < NR; ++i) {
@@ -1107,6 +1118,7 @@ __global__ void __launch_bounds__(kRT, 1)
       const int r = t.rb + i, y = t.y0 + r;
       const int64_t o = (int64_t)y * pitch + t.xa;
       float2 xa, xb2;
+      __syncwarp();
       tmem_ld4(tm + kTRow * i + kTc, xa, xb2);
       tmem_wait_ld();
       tmem_arrived(xa, xb2);
@@ -1162,6 +1174,7 @@ __global__ void __launch_bounds__(kRT, 1)
     if (tid == 0) st_release(done + cta, ord + 1);
   }
   __syncthreads();
+  __syncwarp();
   if (wid == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase),
                  "r"(kCols));
@@ -1216,8 +1229,8 @@ ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag,
       const int tr = (shapes[i].h + nv - 1) / nv;
       rows = std::max(rows, tr);
       fits = tr <= max_rows;
-      // a sweep costs its exchange plus its rows (us, measured: 3.5 at 25 rows, 4.1 at
-      // 41, 4.8 at 61, 5.6 at 81, 6.2 at 97)
+      // a sweep costs its exchange plus its rows (us, measured: 3.6 at 21 rows, 4.1 at
+      // 41, 4.6 at 61, 5.4 at 81, 6.0 at 97)
       const double sweep = 3.0 + 0.033 * tr;
       cost[i] = shapes[i].n_outer * (shapes[i].n_inner + 3.0) * sweep + 5.0;
     }
