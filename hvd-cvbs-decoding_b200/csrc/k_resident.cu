@@ -1106,7 +1106,10 @@ __global__ void __launch_bounds__(kRT, 1)
         }
       }
       // u and y are rewritten by the next pass; every thread is past its
-      // reads of them (the barrier after the sums)
+      // reads of them (the barrier after the sums). No wait of the next pass may
+      // run out before all have read that none had: the warps leave (and free the
+      // tensor memory) together or not at all.
+      __syncthreads();
     }
     if (bad) {
       if (tid == 0) atomicOr(A.err, 1);
