@@ -2,7 +2,7 @@
 //
 // Same iteration as k_solver.cu (VariationalRefine, hvd-core/src/engine/
 // variational.cpp:198-556, with the single-reduction recurrence described
-// there) for fields that fit in the SMs' registers and shared memory. The
+// there) for fields that fit in the SMs' tensor and shared memory. The
 // streaming kernel moves ~82 B of HBM or L2 per pixel in every CG iteration
 // and passes the phases of a lone field through a work queue; here a gang of
 // CTAs takes a whole field, each CTA keeps one tile of it (a 64-column strip
