@@ -168,7 +168,7 @@ struct Smem {
   double* res;          // kNV x collecting warps
   Scalars* sc;
   int* word;            // [0]: a wait ran out, [1..2]: next field
-  static size_t bytes(int rows) {
+  static constexpr size_t bytes(int rows) {
     return (size_t)(rows + 2) * kUB + (size_t)rows * kWB + kStrip * 8 +
            sizeof(double) * (kRW + 5) * kNV + sizeof(Scalars) + 16;
   }
@@ -188,6 +188,21 @@ struct Smem {
     word = reinterpret_cast<int*>(p);
   }
 };
+
+// The tallest tile: kMaxRows, or what fits shared memory beside the fixed part
+// (the neighbour terms take 12 bytes more per pixel: 87 rows).
+constexpr size_t kSmemMax = 232448;
+template <bool kNbr>
+constexpr int tallest_tile() {
+  int rows = kMaxRows;
+  while (Smem<kNbr>::bytes(rows) > kSmemMax) --rows;
+  return rows;
+}
+// Rows per warp of the tallest tile: launch_resident has an instance for each
+// count up to these.
+constexpr int kMaxNr = 7, kMaxNrNbr = 6;
+static_assert(tallest_tile<false>() <= kMaxNr * kRW && tallest_tile<true>() <= kMaxNrNbr * kRW,
+              "an instance for the tallest tile");
 
 __device__ __forceinline__ float4 lds4(uint32_t a) {
   float4 v;
@@ -1189,7 +1204,7 @@ cudaError_t launch_one(const SolverArgs& a, const ResidentPlan& p, cudaStream_t 
   const size_t smem = Smem<kNbr>::bytes(p.rows);
   once([] {
     cudaFuncSetAttribute(k_resident<NR, kNbr>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         232448);
+                         (int)kSmemMax);
   });
   SolverArgs sa = a;
   ResidentArgs ra;
@@ -1212,10 +1227,7 @@ size_t resident_xchg_bytes(int sm_count) {
 ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag, int sm_count) {
   ResidentPlan best;
   if (diag || n <= 0) return best;
-  // rows that fit beside the fixed part (neighbour terms: 12 B more per pixel)
-  int max_rows = kMaxRows;
-  while (max_rows > 0 && (nbr ? Smem<true>::bytes(max_rows) : Smem<false>::bytes(max_rows)) > 232448)
-    --max_rows;
+  const int max_rows = nbr ? tallest_tile<true>() : tallest_tile<false>();
   double best_t = 0.0;
   std::vector<double> cost(n), load;
   for (int g = 1; g <= std::min(n, sm_count); ++g) {
@@ -1264,14 +1276,17 @@ cudaError_t launch_resident(const SolverArgs& a, const ResidentPlan& p, bool nbr
     if (p.nr <= 1) return launch_one<1, true>(a, p, st);
     if (p.nr <= 2) return launch_one<2, true>(a, p, st);
     if (p.nr <= 3) return launch_one<3, true>(a, p, st);
-    return launch_one<5, true>(a, p, st);
+    if (p.nr <= 5) return launch_one<5, true>(a, p, st);
+    if (p.nr <= kMaxNrNbr) return launch_one<kMaxNrNbr, true>(a, p, st);
+    return cudaErrorInvalidValue;
   }
   if (p.nr <= 1) return launch_one<1, false>(a, p, st);
   if (p.nr <= 2) return launch_one<2, false>(a, p, st);
   if (p.nr <= 3) return launch_one<3, false>(a, p, st);
   if (p.nr <= 4) return launch_one<4, false>(a, p, st);
   if (p.nr <= 5) return launch_one<5, false>(a, p, st);
-  return launch_one<7, false>(a, p, st);
+  if (p.nr <= kMaxNr) return launch_one<kMaxNr, false>(a, p, st);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace hvdg
