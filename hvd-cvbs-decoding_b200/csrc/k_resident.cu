@@ -31,9 +31,12 @@
 //    CTAs; a gang's first CTA fetches its next field when all have finished
 //    with the last one.
 //
-// All waits are bounded (SolverArgs::phase_wait_limit polls); a CTA that
-// gives up sets the error flag and leaves, and its peers follow by their own
-// limits. The launch is cooperative, so all CTAs are co-resident.
+// All waits are bounded: SolverArgs::phase_wait_limit polls for what another CTA
+// publishes next. A CTA that has no tile of its gang's field waits for the
+// whole field and takes one such limit for each of the field's exchanges. A CTA
+// that gives up sets the error flag and leaves, its peers follow by their own
+// limits, and a gang's first CTA tells the waiting ones as it leaves. The launch is
+// cooperative, so all CTAs are co-resident.
 //
 // Per-pixel arithmetic, its order and the FP32 row terms of the inner
 // products are those of k_solver.cu; only the order of the FP64 additions
@@ -525,6 +528,7 @@ __global__ void __launch_bounds__(kRT, 1)
   const uint32_t tbase = (uint32_t)M.word[3];
   const uint32_t tm = tbase + ((uint32_t)(wid & 3) << 21) + (uint32_t)(wid >> 2) * (NR * kTRow);
   int prev_parts = 0;  // CTAs of the gang's previous field (first CTA only)
+  long long limits = 1;  // wait limits that the fetch of the next field may take
   for (int ord = 0;; ++ord) {
     int idx = gang;
     if (ord > 0) {
@@ -555,6 +559,8 @@ __global__ void __launch_bounds__(kRT, 1)
           ld_slot(fetch, lo, hi);
           if (hi >= (unsigned long long)ord) break;
           if (++n > A.phase_wait_limit) {
+            n = 0;
+            if (--limits > 0) continue;
             M.word[0] = 1;
             lo = (unsigned long long)A.n_fields;
             hi = (unsigned long long)ord;
@@ -583,7 +589,11 @@ __global__ void __launch_bounds__(kRT, 1)
     nv = (fh + trows - 1) / trows;
     const int parts = ns * nv;
     prev_parts = parts;
-    if (cta >= parts) continue;
+    limits = 1;
+    if (cta >= parts) {
+      limits += f.n_outer * (f.n_inner + 3LL);
+      continue;
+    }
     Tile t;
     {
       const int v = cta / ns, s = cta - v * ns;
@@ -1127,7 +1137,11 @@ __global__ void __launch_bounds__(kRT, 1)
       __syncthreads();
     }
     if (bad) {
-      if (tid == 0) atomicOr(A.err, 1);
+      if (tid == 0) {
+        atomicOr(A.err, 1);
+        // no field follows: the CTAs without a tile need not wait for one
+        if (cta == 0) st_slot(fetch, (unsigned long long)A.n_fields, (unsigned long long)ord + 1);
+      }
       break;
     }
     // ---- F: apply the pending step, luma = S - Re[chi c], outputs ----

@@ -237,7 +237,10 @@ hvdg_status hvdg_set_batching(hvdg_ctx* ctx, int batched);
 hvdg_status hvdg_set_tuning(hvdg_ctx* ctx, int band_rows, int ctas_per_sm);
 /* Bound of the solvers' device-side waits (on a field's phase flag, or on another
  * CTA's part of an exchange), in polls
- * (~0.5 us each; <= 0 restores the default 4,000,000, ~2 s). A wait that
+ * (~0.5 us each; <= 0 restores the default 4,000,000, ~2 s). Where a launch holds
+ * more fields than it solves at a time, a CTA without a part in the current one
+ * waits for it to end: one such bound for each of that field's exchanges (three
+ * and its CG iterations per outer iteration). A wait that
  * runs out ends the launch and the call returns HVDG_ERR_DEVICE_TIMEOUT; the
  * context stays usable. No reference counterpart (the reference's CPU loops
  * have no waits to bound). */
