@@ -1280,6 +1280,7 @@ ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag,
       best.rows = rows;
     }
   }
+  best.us = best_t;
   if (best.gangs) best.nr = (best.rows + kRW - 1) / kRW;
   return best;
 }

@@ -62,6 +62,7 @@ struct SolveShape {
 // the streaming solver takes them.
 struct ResidentPlan {
   int gangs = 0, ctas = 0, rows = 0, nr = 0;
+  double us = 0.0;  // estimated time of the launch
 };
 ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag, int sm_count);
 size_t resident_xchg_bytes(int sm_count);

@@ -201,8 +201,8 @@ struct Layout {
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// Planes of one size, solved by one resident launch: `n` entries of the order
-// table from `off` on.
+// Planes solved by one resident launch: `n` entries of the order table from
+// `off` on.
 struct ResidentGroup {
   hvdg::ResidentPlan plan;
   int off, n;
@@ -227,7 +227,7 @@ struct Batch {
   // per field: the solver writes luma / chroma straight to the caller's
   // buffers (FieldDesc out_y / out_c), so no copy follows
   std::vector<char> direct_y, direct_c;
-  std::vector<int> order;    // planes by size, then by solver work, heaviest first
+  std::vector<int> order;    // the planes of one launch after the other, heaviest first
   std::vector<ResidentGroup> rg;  // empty: the streaming solver takes the batch
   Layout L;
   int max_phases = 0;
