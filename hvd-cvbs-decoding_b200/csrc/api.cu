@@ -137,6 +137,11 @@ hvdg_status hvdg_create(int device, hvdg_ctx** out) {
   hvdg::solver_max_blocks_per_sm();
   hvdg::configure_prep_kernels();
   hvdg::configure_init_kernels();
+  if (hvdg::configure_resident_kernels() != cudaSuccess) {
+    cudaGetLastError();
+    hvdg_destroy(ctx);
+    return HVDG_ERR_CUDA;
+  }
   *out = ctx;
   return HVDG_OK;
 }

@@ -50,7 +50,6 @@
 
 #include "hvdg_common.cuh"
 #include "k_solver.h"
-#include "per_device.h"
 
 namespace hvdg {
 
@@ -1212,14 +1211,20 @@ __global__ void __launch_bounds__(kRT, 1)
                  "r"(kCols));
 }
 
+template <bool kNbr, int... NR>
+cudaError_t configure() {
+  cudaError_t e = cudaSuccess;
+  ((e = e != cudaSuccess ? e
+                         : cudaFuncSetAttribute(k_resident<NR, kNbr>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)kSmemMax)),
+   ...);
+  return e;
+}
+
 template <int NR, bool kNbr>
 cudaError_t launch_one(const SolverArgs& a, const ResidentPlan& p, cudaStream_t st) {
-  static PerDeviceOnce once;
   const size_t smem = Smem<kNbr>::bytes(p.rows);
-  once([] {
-    cudaFuncSetAttribute(k_resident<NR, kNbr>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemMax);
-  });
   SolverArgs sa = a;
   ResidentArgs ra;
   ra.gangs = p.gangs;
@@ -1231,6 +1236,11 @@ cudaError_t launch_one(const SolverArgs& a, const ResidentPlan& p, cudaStream_t 
 }
 
 }  // namespace
+
+cudaError_t configure_resident_kernels() {
+  const cudaError_t e = configure<false, 1, 2, 3, 4, 5, kMaxNr>();
+  return e != cudaSuccess ? e : configure<true, 1, 2, 3, 5, kMaxNrNbr>();
+}
 
 size_t resident_xchg_bytes(int sm_count) {
   // edge and reduction slots per CTA, a fetch slot per gang, a counter per CTA

@@ -65,6 +65,9 @@ struct ResidentPlan {
   double us = 0.0;  // estimated time of the launch
 };
 ResidentPlan plan_resident(const SolveShape* shapes, int n, bool nbr, bool diag, int sm_count);
+// The kernels' attributes on the current device: before the first launch there,
+// outside any stream capture.
+cudaError_t configure_resident_kernels();
 size_t resident_xchg_bytes(int sm_count);
 cudaError_t launch_resident(const SolverArgs& args, const ResidentPlan& plan, bool nbr,
                             cudaStream_t st);
