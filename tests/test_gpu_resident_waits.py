@@ -24,3 +24,23 @@ def test_wait_bound_is_per_exchange():
         got = ctx.decode_fields(fields, cfg)
     for a, b in zip(got, want):
         assert np.array_equal(a.luma, b.luma) and np.array_equal(a.chroma, b.chroma)
+
+
+def test_waits_that_run_out_end_every_gang():
+    """With a bound of one poll the gangs give up in their first exchanges, and
+    their CTAs without a tile with them; the context decodes again afterwards."""
+    g = _cabi.default_geometry(_cabi.STD_NTSC)
+    fields = [api.Field(synth.make_field(80 + i, g.standard, 0.7, field_index=i).samples, g,
+                        parity=i % 2) for i in range(5)]
+    cfg = api.default_config(fast=0, cg_tol=1e-6, temporal_strength=-1.0, irls_outer=2,
+                             cg_iterations=20)
+    with api.Context(0) as ctx:
+        want = ctx.decode_fields(fields, cfg)
+        ctx.set_device_wait_limit(1)
+        with pytest.raises(api.HvdgError) as err:
+            ctx.decode_fields(fields, cfg)
+        assert err.value.status == _cabi.ERR_DEVICE_TIMEOUT
+        ctx.set_device_wait_limit(0)
+        again = ctx.decode_fields(fields, cfg)
+    for a, b in zip(again, want):
+        assert np.array_equal(a.luma, b.luma) and np.array_equal(a.chroma, b.chroma)
