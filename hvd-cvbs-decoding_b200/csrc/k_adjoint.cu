@@ -99,7 +99,7 @@ __global__ void k_adj_norm(AdjGeom g, const float2* __restrict__ chib, double* _
     v[0] = (double)a.x * a.x + (double)a.y * a.y;
   }
   block_sum<1>(v, sh);
-  if (threadIdx.x == 0 && threadIdx.y == 0) 
+  if (threadIdx.x == 0 && threadIdx.y == 0)
     part[(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = v[0];
 }
 
@@ -338,7 +338,7 @@ __global__ void k_adj_samples(AdjGeom g, const AdjField* __restrict__ fields,
   if (x >= fw || y >= fh) return;
   const int ay = y - fal, ax = x - a0;
   float v = 0.f;
-  if (ay >= 0 && ay < g.h && ax >= 0 && ax < g.w) 
+  if (ay >= 0 && ay < g.h && ax >= 0 && ax < g.w)
     v = sbar[plane_of(g) + (int64_t)ay * g.pitch + ax] * fields[blockIdx.z].inv_cpi;
   out[((int64_t)blockIdx.z * fh + y) * fw + x] = v;
 }

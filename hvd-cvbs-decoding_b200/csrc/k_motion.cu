@@ -12,10 +12,11 @@
 // FMA contraction off (--fmad=false), every float / double operation is
 // issued in the reference's order, and each (pair, tile) visits the
 // candidates in the reference's centre-out order with the same
-// partial-distortion bail-out and strict-less update (one thread per tile,
-// or for the refinement a warp per tile that replays the visit from
-// per-row running sums), so the selected vectors, sub-pel fits and
-// confidences equal the reference's bit for bit.
+// partial-distortion bail-out and strict-less update (a block per tile forms the
+// per-row running sums of all candidates and a warp replays the visit from them;
+// searches and tiles past the staged sizes take one thread per tile), so the
+// selected vectors, sub-pel fits and confidences equal the reference's bit for
+// bit.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -1156,9 +1157,9 @@ __global__ void __launch_bounds__(kSadThreads, 6) k_sad_search(const MeField* __
 // the middle ones it finds (750 tiles: 63 us by one CTA in two passes over the
 // ranks, 23 by one of 1024 threads in one pass, 14 by the cluster).
 constexpr int kSadConfThreads = 256, kSadConfCtas = 8;
-__global__ void __cluster_dims__(kSadConfCtas, 1, 1) __launch_bounds__(kSadConfThreads) k_sad_confidence(const MeField* __restrict__ mf,
-                                                        const MePair* __restrict__ pairs,
-                                                        SadArgs a, SadBuffers out) {
+__global__ void __cluster_dims__(kSadConfCtas, 1, 1) __launch_bounds__(kSadConfThreads)
+    k_sad_confidence(const MeField* __restrict__ mf, const MePair* __restrict__ pairs, SadArgs a,
+                     SadBuffers out) {
   extern __shared__ double sadc_sm[];
   __shared__ double mid[2];
   const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -1221,7 +1222,8 @@ void launch_motion_sad(const MeField* d_fields, int nf, int max_h, int max_w,
     cudaFuncSetAttribute(k_sad_search, cudaFuncAttributeMaxDynamicSharedMemorySize, kSadMaxSmem);
   });
   k_sad_search<<<dim3(th * tw, npairs), kSadThreads, smem, st>>>(d_fields, d_pairs, b.qblur, a, b);
-  k_sad_confidence<<<npairs * kSadConfCtas, kSadConfThreads, th * tw * (int)sizeof(double), st>>>(d_fields, d_pairs, a, b);
+  k_sad_confidence<<<npairs * kSadConfCtas, kSadConfThreads, th * tw * (int)sizeof(double), st>>>(
+      d_fields, d_pairs, a, b);
 }
 
 // ---------------------------------------------------------------------------

@@ -132,12 +132,12 @@ __device__ void tridiag_smooth(const double* d, const double* a, int n, double l
 
 // One CTA per field: a line per thread in the smoother and the angles, four
 // lines per warp in the burst sums (256 threads and a line per warp at a time:
-// 67 us for an NTSC field, 100 for PAL; 47 and 62 now, the FP64 divisions of the reduction's 18
-// steps and the angles' FP64 functions bounding it).
+// 67 us for an NTSC field, 100 for PAL; 47 and 62 now, the FP64 divisions of the
+// reduction's 18 steps and the angles' FP64 functions bounding it).
 constexpr int kLkThreads = 512;
 constexpr int kLkLines = 4;
-__global__ void __launch_bounds__(kLkThreads) k_burst_lockin(const PrepDesc* __restrict__ descs,
-                                                      LockinOut out) {
+__global__ void __launch_bounds__(kLkThreads)
+    k_burst_lockin(const PrepDesc* __restrict__ descs, LockinOut out) {
   const PrepDesc p = descs[blockIdx.x];
   const int h = p.fh;
   extern __shared__ double lk_smem[];

@@ -77,9 +77,8 @@ struct __align__(16) Slot {
 };
 constexpr uint32_t kSetBytes = sizeof(Slot) * kOutSlots;
 
-// Exchange memory: per CTA three sets of edge slots, then per CTA two sets of
-// reduction slots (laid out value-major inside a gang), then a fetch slot and
-// a done counter per CTA.
+// Exchange memory: per CTA three sets of edge slots, then per gang the sum slots
+// ([set][copy][CTA][value]), then a fetch slot per gang and a done counter per CTA.
 __host__ __device__ constexpr size_t edge_bytes() { return sizeof(Slot) * kSets * kOutSlots; }
 __host__ __device__ constexpr size_t red_bytes() { return sizeof(Slot) * 2 * kLine * kRep; }
 
@@ -759,7 +758,9 @@ __global__ void __launch_bounds__(kRT, 1)
         tmem_wait_st();
         if (hrole) {
           unsigned long long lo;
-          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo, A.phase_wait_limit)) M.word[0] = 1;
+          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo,
+                         A.phase_wait_limit))
+            M.word[0] = 1;
           const float2 hx = unpack2(lo);
           sts2(hu, hx);
           sts1(hyp, hS - re_rn(hx, hc));
@@ -875,13 +876,15 @@ __global__ void __launch_bounds__(kRT, 1)
         // the row above's vertical weights, the left column's horizontal ones
         if (hrole && (tid < kStrip || (tid >= 2 * kStrip && tid < 2 * kStrip + kSideCap))) {
           unsigned long long lo;
-          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo, A.phase_wait_limit)) M.word[0] = 1;
+          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo,
+                         A.phase_wait_limit))
+            M.word[0] = 1;
           const float2 w2 = unpack2(lo);
           sts2(tid < kStrip ? M.wtop + 8 * tid : M.u + (tid - 2 * kStrip + 1) * kUB + kWL, w2);
         }
       }
       __syncthreads();
-      // ---- G: the gradient at chi into registers ----
+      // ---- G: the gradient at chi into tensor memory ----
       ++ex;
       set = set == kSets - 1 ? 0 : set + 1;
       double pgg0 = 0.0;
@@ -923,7 +926,9 @@ __global__ void __launch_bounds__(kRT, 1)
         tmem_wait_st();
         if (hrole) {
           unsigned long long lo;
-          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo, A.phase_wait_limit)) M.word[0] = 1;
+          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo,
+                         A.phase_wait_limit))
+            M.word[0] = 1;
           hg = unpack2(lo);
           hd = make_float2(-hg.x, -hg.y);
         }
@@ -1060,7 +1065,9 @@ __global__ void __launch_bounds__(kRT, 1)
         float2 hq = z;
         if (hrole) {
           unsigned long long lo;
-          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo, A.phase_wait_limit)) M.word[0] = 1;
+          if (!poll_slot(reinterpret_cast<const Slot*>(xb + hsrc + set * kSetBytes), tag, lo,
+                         A.phase_wait_limit))
+            M.word[0] = 1;
           hq = unpack2(lo);
         }
         if (wid >= kRedWarp0) {

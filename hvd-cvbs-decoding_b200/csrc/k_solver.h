@@ -29,7 +29,7 @@ struct SolverArgs {
   int* garrive;                 // per unit group (slot unit_begin + group), 0 before launch
   double* gpartials;            // per unit group x 5 (same slots)
   int* err;                     // set on a bounded-wait timeout
-  long long phase_wait_limit;   // polls of a field's phase flag before giving up (err)
+  long long phase_wait_limit;   // polls of a phase flag or of an exchange before giving up (err)
   const float* S;
   float2* X[2];                 // chi (double-buffered; final chi in X[0])
   float2* G[2];
@@ -47,7 +47,7 @@ struct SolverArgs {
   // the resident solver (k_resident.cu)
   const int* order;             // this launch's fields, heaviest first
   int n_fields;
-  void* xchg;                   // kResidentXchgBytes(sm_count), zeroed before launch
+  void* xchg;                   // resident_xchg_bytes(CTAs of the launch), zeroed before it
   int keep_w;                   // the last outer's weights are also left in W
 };
 

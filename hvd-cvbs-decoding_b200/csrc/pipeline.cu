@@ -410,7 +410,7 @@ hvdg_status plan_batch(hvdg_ctx* ctx, const hvdg_field_in* in, int n, const hvdg
     ncol += t.w;
   }
   // the resident solver wherever the planes fit (a tiling set by the caller
-  // or the tuner belongs to the streaming one); it takes no units
+  // or the tuner belongs to the streaming one); it does not use the units below
   const std::vector<hvdg::SolveShape> shapes = solve_shapes(in, n, cfg, weave_geom);
   b.order.assign(m, 0);
   if (resident_allowed(ctx, band_rows))

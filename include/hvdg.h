@@ -450,6 +450,9 @@ hvdg_status hvdg_verify_motion(hvdg_ctx* ctx, const float* y_ref, const float* y
  * converges every outer. Held at their forward values (no gradient through
  * them): the lock-in carrier phase and the chroma-anisotropy split; samples
  * outside the active window therefore get zero gradient.
+ * Consecutive fields of one geometry and budget go through together, up to 32 or
+ * as many as 4 GB of device memory hold (one at a time where there is less); the
+ * context keeps that memory, as after any call, until it is destroyed.
  * out (optional, may be NULL): the recomputed forward's luma / chroma. */
 hvdg_status hvdg_decode_fields_adjoint(hvdg_ctx* ctx, const hvdg_field_in* fields, int n,
                                        const hvdg_config* cfg, const float* const* y_bar,

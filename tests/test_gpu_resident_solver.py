@@ -1,7 +1,7 @@
 """The resident solver (k_resident.cu) against the streaming one (k_solver.cu)
 and the FP64 oracle, where its tiling can go wrong: planes narrower than a
-strip, one column or row past a tile, odd widths, fewer rows than warps, the
-tallest tile (97 rows), more fields than gangs, mixed sizes in one batch, the
+strip, one column or row past a tile, odd widths, fewer rows than warps,
+tall tiles (97 rows), more fields than gangs, mixed sizes in one batch, the
 3-D neighbour terms, and a pass that ends early.
 
 The two kernels perform the same operations on every pixel and differ only in
